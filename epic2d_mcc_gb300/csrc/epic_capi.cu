@@ -418,7 +418,9 @@ epic_status do_solve(epic_sim* s) {
   } else {
     const int nb = s->cfg.solver_blocks > 0 ? std::min(s->cfg.solver_blocks, solver_max_blocks())
                                             : pcg_default_blocks(nnodes(s), s->num_sms);
-    launch_pcg(s->stream, a, nb);
+    s->launches += launch_pcg(s->stream, a, nb);
+    CKL();
+    return EPIC_OK;
   }
   s->launches += s->cfg.poisson_bc != EPIC_POISSON_DIRICHLET ? 2 : 1;  // + the duplicated nodes' fill
   CKL();

@@ -1455,864 +1455,24 @@ int solver_max_blocks() {
   return v;
 }
 
-// ------------------------------------------------------ tiled PCG ---
-// The same Chronopoulos-Gear iteration as k_pcg, with the unknowns held in
-// registers for the whole solve.  The lattice of unknowns (R = ny rows of
-// C = nx columns, row = k / nx as in the reference's dense A) is cut into
-// one tr x tc tile per CTA; each thread owns up to NPT nodes of its tile and
-// keeps their x, r, w, p, s in registers.  The stencil reads r from a
-// shared-memory copy of the tile with a one-node halo ring: halo nodes belong
-// to neighbouring tiles, whose owners publish r, w, s of their edge nodes
-// (double-buffered by iteration parity) before the grid barrier, so after it
-// each CTA recomputes the halo's new r - alpha(w + beta s) from them.
-//
-// Exact identities of the constant Jacobi diagonal -4 remove M from the
-// loop: with u = M r = -r/4 every product with u is an exact power-of-two
-// scaling, so w = A u = fma(-1/4, sum of the neighbours' r, r), (w, u) =
-// -(w, r)/4, gamma = (r, u) = -(r, r)/4, and p is kept as p' = -4p (p' = r +
-// beta p', x += (-alpha/4) p').  All of these round exactly as the unscaled
-// forms do.  That leaves 10 FP64 operations per node and iteration, and the
-// p'/x updates (needed only for the answer) run while the CTA waits at the
-// grid barrier, so 8 are on the critical path.  The iteration's scalars need
-// one division there: beta = gamma * (1/gamma_prev), with the reciprocal
-// formed while waiting, and eta = delta - beta*gamma/alpha_prev =
-// delta - beta^2 eta_prev (alpha_prev = gamma_prev/eta_prev), formed as
-// delta - gamma^2 (eta_prev/gamma_prev^2) with the second factor also formed
-// while waiting; alpha = gamma/eta by div_nr.
-//
-// One grid-wide synchronisation per iteration carries both dot products: the
-// CTAs add their fixed-point partials into counted words of a slot (see
-// PCG_SLOT_WORDS), so the poll that ends the barrier also returns the totals.
-// The first iteration, and any whose terms outgrow the anchors, reduce
-// through block-anchored partials and the counter barrier instead.
-struct PcgTiling {
-  int tr, tc;          // tile rows, columns
-  int tiles_c;         // tiles per lattice row
-  int blocks;          // CTAs (tiles)
-  int npt;             // owned-node slots per thread
-};
-
-constexpr int PCG_T = 256;
-constexpr int PCG_HALO_SLOTS = 2;    // halo nodes per thread (the halo ring holds <= 512)
-constexpr int PCG_MAX_BLOCKS = 160;  // partial records read per lane: PCG_MAX_BLOCKS / 32
-
-// Split grid barrier: each CTA counts its own barrier episodes, so arriving
-// needs no returned ticket (a fire-and-forget red.release by thread 0 after a
-// __syncthreads that orders the block's writes before it), and work that no
-// other CTA needs can run between arriving and waiting.
-__device__ __forceinline__ void bar_arrive(unsigned int* bar) {
-  asm volatile("red.release.gpu.global.add.u32 [%0], %1;" ::"l"(bar), "r"(1u) : "memory");
-}
-
-// Waits until `target` arrivals are in (bounded: FLAG_TIMEOUT and false on
-// giving up).  Ends with a __syncthreads.
-__device__ __forceinline__ bool bar_wait(unsigned int* bar, int* flags, unsigned int target, int* s_ok,
-                                         long long limit) {
-  if (threadIdx.x == 0) {
-    int ok = 1;
-    long long spins = 0;
-    while ((int)(ld_acquire_gpu(bar) - target) < 0) {
-      if (++spins >= limit) {
-        atomicOr(flags, FLAG_TIMEOUT);
-        ok = 0;
-        break;
-      }
-    }
-    *s_ok = ok;
-  }
-  __syncthreads();
-  return *s_ok;
-}
-
-// One CTA's exact partial of two dot products: V = sum * 2^(1129 - a).
-struct XPartial {
-  unsigned long long lo[2];
-  long long hi[2];
-  int a[2];
-  int pad[2];
-};
-
-struct XScratch {
-  int e[2][PCG_T / 32];
-  unsigned long long v[2][PCG_T / 32][2];
-};
-
-// Block partial of the terms t0[j], t1[j] (j < NT) of every thread; thread 0
-// stores it to *out.  Two __syncthreads (anchor exponents, warp totals).
-template <int NT>
-__device__ __forceinline__ void xs_block_partial(const double (&t0)[NT], const double (&t1)[NT], XScratch& sx,
-                                                 XPartial* out) {
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  int e0 = 0, e1 = 0;
-#pragma unroll
-  for (int j = 0; j < NT; j++) {
-    e0 = max(e0, xs_exponent(t0[j]));
-    e1 = max(e1, xs_exponent(t1[j]));
-  }
-  e0 = (int)__reduce_max_sync(0xffffffffu, (unsigned)e0);
-  e1 = (int)__reduce_max_sync(0xffffffffu, (unsigned)e1);
-  if (lane == 0) {
-    sx.e[0][wid] = e0;
-    sx.e[1][wid] = e1;
-  }
-  __syncthreads();
-  int A0 = 0, A1 = 0;
-#pragma unroll
-  for (int w = 0; w < PCG_T / 32; w++) {
-    A0 = max(A0, sx.e[0][w]);
-    A1 = max(A1, sx.e[1][w]);
-  }
-  xs_int v0 = 0, v1 = 0;
-#pragma unroll
-  for (int j = 0; j < NT; j++) {
-    v0 += xs_from_double(t0[j], A0);
-    v1 += xs_from_double(t1[j], A1);
-  }
-  v0 = xs_warp_sum(v0);
-  v1 = xs_warp_sum(v1);
-  if (lane == 0) {
-    sx.v[0][wid][0] = (unsigned long long)(xs_uint)v0;
-    sx.v[0][wid][1] = (unsigned long long)((xs_uint)v0 >> 64);
-    sx.v[1][wid][0] = (unsigned long long)(xs_uint)v1;
-    sx.v[1][wid][1] = (unsigned long long)((xs_uint)v1 >> 64);
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    xs_uint s0 = 0, s1 = 0;
-#pragma unroll
-    for (int w = 0; w < PCG_T / 32; w++) {
-      s0 += ((xs_uint)sx.v[0][w][1] << 64) | sx.v[0][w][0];
-      s1 += ((xs_uint)sx.v[1][w][1] << 64) | sx.v[1][w][0];
-    }
-    XPartial p;
-    p.lo[0] = (unsigned long long)s0;
-    p.hi[0] = (long long)(s0 >> 64);
-    p.lo[1] = (unsigned long long)s1;
-    p.hi[1] = (long long)(s1 >> 64);
-    p.a[0] = A0;
-    p.a[1] = A1;
-    p.pad[0] = p.pad[1] = 0;
-    *out = p;
-  }
-}
-
-// Grid totals of the nb partials, by warp 0 (all loads issued first); the
-// doubles are valid in thread 0.
-__device__ __forceinline__ void xs_grid_totals_w0(const XPartial* Pc, int nb, double* out0, double* out1) {
-  constexpr int Q = PCG_MAX_BLOCKS / 32;
-  ulonglong2 r01[Q], r23[Q];
-  int2 ra[Q];
-#pragma unroll
-  for (int q = 0; q < Q; q++) {
-    const int k = threadIdx.x + 32 * q;
-    if (k < nb) {
-      const ulonglong2* rec = reinterpret_cast<const ulonglong2*>(Pc + k);
-      r01[q] = __ldcg(rec);
-      r23[q] = __ldcg(rec + 1);
-      ra[q] = __ldcg(reinterpret_cast<const int2*>(rec + 2));
-    } else {
-      r01[q] = make_ulonglong2(0, 0);
-      r23[q] = make_ulonglong2(0, 0);
-      ra[q] = make_int2(0, 0);
-    }
-  }
-  int a0 = 0, a1 = 0;
-#pragma unroll
-  for (int q = 0; q < Q; q++) {
-    a0 = max(a0, ra[q].x);
-    a1 = max(a1, ra[q].y);
-  }
-  const int A0 = (int)__reduce_max_sync(0xffffffffu, (unsigned)a0);
-  const int A1 = (int)__reduce_max_sync(0xffffffffu, (unsigned)a1);
-  xs_int s0 = 0, s1 = 0;
-#pragma unroll
-  for (int q = 0; q < Q; q++) {
-    // record layout: lo[0], lo[1] | hi[0], hi[1] | a[0], a[1]
-    const xs_int v0 = (xs_int)(((xs_uint)r23[q].x << 64) | r01[q].x);
-    const xs_int v1 = (xs_int)(((xs_uint)r23[q].y << 64) | r01[q].y);
-    s0 += xs_realign(v0, ra[q].x, A0);
-    s1 += xs_realign(v1, ra[q].y, A1);
-  }
-  s0 = xs_warp_sum(s0);
-  s1 = xs_warp_sum(s1);
-  // Lanes 0 and 1 round one total each, side by side.
-  const double d = xs_to_double(threadIdx.x == 0 ? s0 : s1, threadIdx.x == 0 ? A0 : A1);
-  const double d1 = __shfl_sync(0xffffffffu, d, 1);
-  if (threadIdx.x == 0) {
-    *out0 = d;
-    *out1 = d1;
-  }
-}
-
-// 1/x by Newton-Raphson (y <- y + y(1 - m y), two steps) on the significand m
-// of x, seeded with the FP32 reciprocal of m's leading 24 bits: the ~2^-23
-// seed error squares to below FP64 rounding, so the result is within about
-// one ulp of 1/x (not correctly rounded).  The exponent is applied in the
-// integer domain.  Four dependent FP64 operations in all, against a library
-// division's longer sequence; for x and 1/x in the normal range (otherwise
-// the library division is used).
-__device__ __forceinline__ double recip_nr(double x) {
-  const uint64_t b = xs_bits(x);
-  const int e = (int)((b >> 52) & 0x7FF);
-  const uint64_t sign = b & (1ull << 63);
-  if (e == 0 || e >= 2046) return 1.0 / x;
-  const double m = xs_double((b & 0xFFFFFFFFFFFFFull) | (1023ull << 52));  // |x| scaled to [1, 2)
-  const float mf = __int_as_float(0x3F800000 | (int)((b >> 29) & 0x7FFFFF));
-  const float yf = __frcp_rn(mf);  // in (0.5, 1]
-  const unsigned yb = (unsigned)__float_as_int(yf);
-  double y = xs_double(((uint64_t)(((yb >> 23) & 0xFF) - 127 + 1023) << 52) | ((uint64_t)(yb & 0x7FFFFF) << 29));
-  double t = fma(-m, y, 1.0);
-  y = fma(y, t, y);
-  t = fma(-m, y, 1.0);
-  y = fma(y, t, y);
-  const uint64_t rb = xs_bits(y);
-  const long er = (long)((rb >> 52) & 0x7FF) + 1023 - e;
-  if (er <= 0 || er >= 2047) return 1.0 / x;
-  return xs_double(sign | ((uint64_t)er << 52) | (rb & 0xFFFFFFFFFFFFFull));
-}
-
-// ---- fused grid barrier and reduction ----
-// A slot is PCG_SLOT_WORDS 64-bit words, each on its own 128-byte line so that
-// the CTAs' additions to different words proceed in parallel in L2 instead of
-// queueing on one line.  Every CTA adds
-// (payload << 8) + 1 to each word, so a word whose low byte has reached the
-// CTA count is complete and its upper bits hold the payload total: polling a
-// slot is the barrier and returns the reduction in the same load.  Payloads:
-// the 26-bit limb totals of the CTA's fixed-point partials of (w, r) (words
-// 0-4) and (r, r) (words 5-9) against grid-wide anchors, and whether the CTA
-// had a term beyond the anchors' range (word 10).  Slots rotate over three:
-// iteration k adds to slot k % 3, and once CTA 0 has seen it complete it
-// clears slot (k - 1) % 3 (every CTA read that one before adding to slot k);
-// it is next written in iteration k + 2, after the adders have seen slot
-// k + 1 complete, which includes CTA 0's addition after the clearing.
-constexpr int PCG_SLOT_WORDS = 11;
-constexpr int PCG_WORD_STRIDE = 16;  // 64-bit words: one 128-byte line per slot word
-constexpr int PCG_SLOT_U64 = PCG_SLOT_WORDS * PCG_WORD_STRIDE;
-constexpr int PCG_SLOTS = 3;
-// Byte offset of the slots in the partials buffer (after two parities of
-// XPartial records).
-constexpr size_t PCG_SLOT_OFFSET = 2 * PCG_MAX_BLOCKS * sizeof(XPartial);
-static_assert(PCG_MAX_BLOCKS < 256, "the CTA count must fit the low byte of a slot word");
-static_assert(PCG_SLOT_OFFSET % 128 == 0, "slots are 128-byte lines");
-// The partials buffer holds at least 16 x 320 doubles (epic_create) and the
-// allocation-free entry's 8 x 1024.
-static_assert(PCG_SLOT_OFFSET + PCG_SLOTS * PCG_SLOT_U64 * sizeof(unsigned long long) <= 16 * 320 * sizeof(double),
-              "slots must fit the solver partials buffer");
-// Anchors: (r, r) terms of iteration k+1 are converted against the exponent
-// of (r, r) of iteration k plus this headroom, (w, r) terms one higher
-// (|w_i r_i| <= 2 max r_i^2 for the diagonal -4 stencil).  A term more than
-// one binade above its anchor (a residual component that grew past about
-// 2^4 x the previous (r, r)) sends the iteration through the block-anchored
-// reduction instead.  Below the anchor, bits under 2^(A - 1129) are dropped:
-// about 2^-80 of (r, r) for 2^19 terms, far below FP64 rounding.
-constexpr int PCG_ANCHOR_HEADROOM = 3;
-
-__device__ __forceinline__ void red_add_u64(unsigned long long* p, unsigned long long v) {
-  asm volatile("red.relaxed.gpu.global.add.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
-}
-__device__ __forceinline__ void red_release_add_u64(unsigned long long* p, unsigned long long v) {
-  asm volatile("red.release.gpu.global.add.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
-}
-__device__ __forceinline__ unsigned long long ld_acquire_u64(const unsigned long long* p) {
-  unsigned long long v;
-  asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
-  return v;
-}
-__device__ __forceinline__ unsigned long long ld_relaxed_u64(const unsigned long long* p) {
-  unsigned long long v;
-  asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
-  return v;
-}
-
-// acc += x * 2^(1129 - A) (the fixed-point value of xs_from_double, bits
-// under 2^0 truncated toward zero) for x with biased exponent <= A + 1, branch
-// free; a term above that range adds nothing and returns false.  NONNEG: x is
-// known to be >= 0 (squares), so no conditional negation.
-template <bool NONNEG>
-__device__ __forceinline__ bool xs_add_anchored(xs_uint& acc, double x, int A) {
-  const uint64_t b = xs_bits(x);
-  const int eb = (int)((b >> 52) & 0x7FF);
-  const bool ok = eb <= A + 1;
-  const uint64_t m = ok ? ((b & 0xFFFFFFFFFFFFFull) | ((uint64_t)(eb != 0) << 52)) : 0ull;
-  const int sh = 54 + (eb ? eb : 1) - A;  // <= 55 when ok
-  const unsigned up = (unsigned)max(sh, 0), dn = (unsigned)max(-sh, 0);
-  const uint64_t lo = sh >= 0 ? xs_shl(m, up) : xs_shr(m, dn);
-  const uint64_t hi = xs_shr(m, 64u - up);  // m >> (64 - sh), 0 for sh <= 0
-  xs_uint v = ((xs_uint)hi << 64) | lo;
-  if (!NONNEG) {
-    const xs_uint neg = (xs_uint)(xs_int)(-(int64_t)(b >> 63));  // all ones for a negative x
-    v = (v ^ neg) - neg;
-  }
-  acc += v;
-  return ok;
-}
-
-// Warp totals of the five 26-bit limbs of v (top limb signed), in every lane:
-// v = sum l[k] 2^(26k).  Each limb total of 32 lanes stays below 2^31.
-__device__ __forceinline__ void xs_warp_limbs(xs_int v, int (&l)[5]) {
-  const xs_uint u = (xs_uint)v;
-  const unsigned M = (1u << 26) - 1;
-  l[0] = __reduce_add_sync(0xffffffffu, (int)((unsigned)u & M));
-  l[1] = __reduce_add_sync(0xffffffffu, (int)((unsigned)(u >> 26) & M));
-  l[2] = __reduce_add_sync(0xffffffffu, (int)((unsigned)(u >> 52) & M));
-  l[3] = __reduce_add_sync(0xffffffffu, (int)((unsigned)(u >> 78) & M));
-  l[4] = __reduce_add_sync(0xffffffffu, (int)(v >> 104));
-}
-
-// num / den (den normal, finite) from the FP32 reciprocal y0 of den's
-// significand m: with e = 1 - m y0 (|e| < 2^-22), num/m = num y0 (1 + e + e^2)
-// to a relative 2^-66, formed as fma(q0, fma(e, e, e), q0), q0 = num y0:
-// three dependent FP64 operations after the seed, within about two ulps.
-// The exponent is applied in the integer domain; outside the normal range (or
-// for den not normal) the library division is used.
-__device__ __forceinline__ double div_nr(double num, double den) {
-  const uint64_t b = xs_bits(den);
-  const int e = (int)((b >> 52) & 0x7FF);
-  if (e == 0 || e >= 2046) return num / den;
-  const double m = xs_double((b & 0xFFFFFFFFFFFFFull) | (1023ull << 52));  // |den| scaled to [1, 2)
-  const float yf = __frcp_rn(__int_as_float(0x3F800000 | (int)((b >> 29) & 0x7FFFFF)));
-  const unsigned yb = (unsigned)__float_as_int(yf);
-  const double y0 =
-      xs_double(((uint64_t)(((yb >> 23) & 0xFF) - 127 + 1023) << 52) | ((uint64_t)(yb & 0x7FFFFF) << 29));
-  const double er = fma(-m, y0, 1.0);
-  const double q0 = num * y0;
-  const double q = fma(q0, fma(er, er, er), q0);
-  const uint64_t qb = xs_bits(q);
-  const long eq = (long)((qb >> 52) & 0x7FF);
-  const long en = eq - (e - 1023);
-  if (eq == 0 || eq == 0x7FF || en <= 0 || en >= 2047) return num / den;
-  return xs_double(((qb ^ b) & (1ull << 63)) | ((uint64_t)en << 52) | (qb & 0xFFFFFFFFFFFFFull));
-}
-
-template <int NPT>
-__global__ void __launch_bounds__(PCG_T) k_pcg_tiled(SolverArgs a, PcgTiling t) {
-  extern __shared__ double sr[];  // r of the tile and its halo ring, (tr + 2) x (tc + 2)
-  __shared__ XScratch sx;
-  __shared__ double s_alpha, s_beta;
-  __shared__ int s_done, s_ok;
-  __shared__ double s_mean;
-  const Lattice lat = make_lattice(a.g.nx, a.g.ny, a.poisson_bc);
-  const int C = lat.C, R = lat.R;
-  const int n = C * R;
-  const int tr = t.tr, tc = t.tc, ldu = tc + 2;
-  const int br = blockIdx.x / t.tiles_c, bc = blockIdx.x - br * t.tiles_c;
-  const int r0 = br * tr, c0 = bc * tc;
-  // Valid extent of this tile (the last tile row and column may be partial).
-  const int vr = min(tr, R - r0), vc = min(tc, C - c0);
-  const int nb = gridDim.x;
-  const double dx2 = a.g.dx * a.g.dx;
-  const long long spin = spin_or_default(a.spin);
-  // Partials [2][nb] alternate by reduction parity (a CTA can run at most one
-  // reduction ahead of the slowest reader); published edge values likewise:
-  // work[1|2] = r, work[3|4] = w, work[5|6] = s.
-  XPartial* const P = reinterpret_cast<XPartial*>(a.partials);
-  unsigned int target = 0;
-  int ep = 0;  // episodes of the block-anchored reduction (partials parity)
-  // The right-hand side at node k: the reference's (zero on the grid edges),
-  // or -rho dx^2 K on every unknown of an extension lattice.
-  auto rhs = [&](int k) -> double {
-    if (lat.mode == EPIC_POISSON_DIRICHLET) {
-      const int i = k / a.g.ny;
-      return rhs_at(a, k, i, k - i * a.g.ny, dx2);
-    }
-    return -a.rho[k] * dx2 * a.K;
-  };
-
-  for (int m = threadIdx.x; m < (tr + 2) * ldu; m += PCG_T) sr[m] = 0.0;
-
-  // Edge publication: each tile writes its boundary to an edge buffer of
-  // 2 (tc + tr) slots per tile - top row at 0, bottom row at tc, left column
-  // at 2 tc, right column at 2 tc + tr, the bottom row and right column being
-  // the last valid ones - so that a neighbour reads each side of its halo
-  // ring as one contiguous run (a column of the lattice would be one
-  // scattered load per node).  Tiles span at least 2 x 2 valid nodes where a
-  // neighbour can lie beyond them (pcg_tiling), so a node lies on at most one
-  // row side and one column side.
-  const int ebase = blockIdx.x * 2 * (tc + tr);
-  // Owned slots: tile-local q = threadIdx.x + PCG_T*j, row-major in the tile.
-  int kk[NPT], si[NPT], pe0[NPT], pe1[NPT];
-#pragma unroll
-  for (int j = 0; j < NPT; j++) {
-    const int q = threadIdx.x + PCG_T * j;
-    const int lr = q / tc, lc = q - lr * tc;
-    const int row = r0 + lr, col = c0 + lc;
-    const bool valid = q < tr * tc && row < R && col < C;
-    kk[j] = valid ? lattice_node(lat, row, col) : -1;
-    si[j] = (lr + 1) * ldu + lc + 1;
-    const int er = lr == 0 ? ebase + lc : lr == vr - 1 ? ebase + tc + lc : -1;
-    const int ec = lc == 0 ? ebase + 2 * tc + lr : lc == vc - 1 ? ebase + 2 * tc + tr + lr : -1;
-    pe0[j] = !valid ? -1 : er >= 0 ? er : ec;
-    pe1[j] = !valid || er < 0 ? -1 : ec;
-  }
-  // Halo slots: the ring around the valid extent - above, below, left, right
-  // - with the node (hk, for the set-up) and the neighbour tile's edge slot
-  // (he): the neighbour above publishes its bottom row, the one below its top
-  // row, and so on.  Neighbours wrap around where the lattice is periodic.
-  int hk[PCG_HALO_SLOTS], hs[PCG_HALO_SLOTS], he[PCG_HALO_SLOTS];
-#pragma unroll
-  for (int j = 0; j < PCG_HALO_SLOTS; j++) {
-    const int h = threadIdx.x + PCG_T * j;
-    int row = -1, col = -1, side = -1, sr_ = 0, sc = 0;
-    if (h < vc) {
-      side = 0; row = r0 - 1; col = c0 + h; sr_ = 0; sc = h + 1;
-    } else if (h < 2 * vc) {
-      side = 1; row = r0 + vr; col = c0 + h - vc; sr_ = vr + 1; sc = h - vc + 1;
-    } else if (h < 2 * vc + vr) {
-      side = 2; row = r0 + h - 2 * vc; col = c0 - 1; sr_ = h - 2 * vc + 1; sc = 0;
-    } else if (h < 2 * vc + 2 * vr) {
-      side = 3; row = r0 + h - 2 * vc - vr; col = c0 + vc; sr_ = h - 2 * vc - vr + 1; sc = vc + 1;
-    }
-    if (side >= 0) {
-      row = lattice_wrap(row, R, lat.wrap_r);
-      col = lattice_wrap(col, C, lat.wrap_c);
-    }
-    const bool valid = side >= 0 && row >= 0 && col >= 0;
-    int e = -1;
-    if (valid) {
-      const int nbr = row / tr, nbc = col / tc;
-      const int nlr = row - nbr * tr, nlc = col - nbc * tc;
-      const int eslot = side == 0 ? tc + nlc : side == 1 ? nlc : side == 2 ? 2 * tc + tr + nlr : 2 * tc + nlr;
-      e = (nbr * t.tiles_c + nbc) * 2 * (tc + tr) + eslot;
-    }
-    hk[j] = valid ? lattice_node(lat, row, col) : -1;
-    he[j] = e;
-    hs[j] = sr_ * ldu + sc;
-  }
-
-  // set-up: x = 0, r = b, w = A(M r), p' = s = 0.
-  double x[NPT], r[NPT], w[NPT], p[NPT], s[NPT], r_old[NPT];
-#pragma unroll
-  for (int j = 0; j < NPT; j++) {
-    x[j] = r[j] = w[j] = p[j] = s[j] = r_old[j] = 0.0;
-    if (kk[j] >= 0) r[j] = rhs(kk[j]);
-  }
-  // PERIODIC: b projected onto zero mean (the mean of the exact total,
-  // rounded once; the singular system is then consistent).
-  double bmean = 0.0;
-  if (lat.mode == EPIC_POISSON_PERIODIC) {
-    double t0[NPT], t1[NPT];
-#pragma unroll
-    for (int j = 0; j < NPT; j++) {
-      t0[j] = kk[j] >= 0 ? r[j] : 0.0;
-      t1[j] = 0.0;
-    }
-    XPartial* const Pc = P + (ep & 1) * nb;
-    xs_block_partial<NPT>(t0, t1, sx, Pc + blockIdx.x);
-    if (threadIdx.x == 0) bar_arrive(a.bar);
-    target += nb;
-    if (!bar_wait(a.bar, a.flags, target, &s_ok, spin)) return;
-    if (threadIdx.x < 32) {
-      double tot = 0, unused = 0;
-      xs_grid_totals_w0(Pc, nb, &tot, &unused);
-      if (threadIdx.x == 0) s_mean = tot / (double)n;
-    }
-    ep++;
-    __syncthreads();
-    bmean = s_mean;
-#pragma unroll
-    for (int j = 0; j < NPT; j++)
-      if (kk[j] >= 0) r[j] = r[j] - bmean;
-  }
-#pragma unroll
-  for (int j = 0; j < NPT; j++)
-    if (kk[j] >= 0) sr[si[j]] = r[j];
-#pragma unroll
-  for (int j = 0; j < PCG_HALO_SLOTS; j++)
-    if (hk[j] >= 0) sr[hs[j]] = rhs(hk[j]) - bmean;
-  __syncthreads();
-  // Dot-product terms of this thread's nodes: (w, r) and (r, r).
-  double td[NPT], tq[NPT];
-#pragma unroll
-  for (int j = 0; j < NPT; j++) {
-    td[j] = tq[j] = 0.0;
-    if (kk[j] >= 0) {
-      const double* c = sr + si[j];
-      w[j] = fma(-0.25, (c[-ldu] + c[-1]) + (c[1] + c[ldu]), r[j]);
-      td[j] = w[j] * r[j];
-      tq[j] = r[j] * r[j];
-      if (pe0[j] >= 0) {
-        a.work[1][pe0[j]] = r[j];
-        a.work[3][pe0[j]] = w[j];
-        a.work[5][pe0[j]] = 0.0;
-      }
-      if (pe1[j] >= 0) {
-        a.work[1][pe1[j]] = r[j];
-        a.work[3][pe1[j]] = w[j];
-        a.work[5][pe1[j]] = 0.0;
-      }
-    }
-  }
-
-  // min(n*n, max_iteration) as pcg() caps it: n*n in 32-bit int arithmetic for
-  // the reference's lattice (it wraps, as there), in 64 bits for the extensions.
-  unsigned int cap32 = (unsigned int)n * (unsigned int)n;
-  const long long cap = lat.mode == EPIC_POISSON_DIRICHLET ? (long long)(int)cap32 : (long long)n * n;
-  const int maxit = cap < a.max_iter ? (int)cap : a.max_iter;
-  unsigned long long* const slots =
-      reinterpret_cast<unsigned long long*>(reinterpret_cast<char*>(a.partials) + PCG_SLOT_OFFSET);
-  // The counted sums hold up to 2^19 terms (the fixed-point headroom).
-  const bool fused = n < (1 << 19);
-  if (blockIdx.x == 0)
-    for (int m = threadIdx.x; m < PCG_SLOTS * PCG_SLOT_U64; m += PCG_T) slots[m] = 0ull;
-  __shared__ int s_limb[PCG_T / 32][PCG_SLOT_WORDS];
-  __shared__ int s_aq, s_exact;
-  // Thread 0's scalars, in the scaled form: rr = (r, r) = -4 gamma,
-  // dr = (w, r) = -4 delta, eta_r = -4 eta; then beta = rr / rr_prev,
-  // eta_r = dr - beta^2 eta_r_prev = dr - rr^2 g with g = eta_r_prev / rr_prev^2,
-  // alpha = rr / eta_r.  Thread 32 forms 1/rr_prev and g while the CTA waits.
-  __shared__ double s_rr, s_eta, s_rrinv, s_g;
-  if (threadIdx.x == 0) s_rr = s_eta = s_rrinv = s_g = 0.0;
-  double be = 0, alq = 0;  // this iteration's beta and -alpha/4
-  int aq = 0;              // anchor of the (r, r) terms (grid-wide); (w, r) one higher
-  int it = 0;
-  // This thread's fixed-point sums of its (w, r) and (r, r) terms against the
-  // anchors, accumulated as the stencil forms the terms.
-  xs_uint v0 = 0, v1 = 0;
-  bool in = true;
-  for (;;) {
-    const int cur = it & 1;
-    double dr = 0, rr = 0;  // valid in thread 0
-    bool exact = it == 0 || !fused;
-    if (!exact) {
-      // Counted sums against the anchors aq (r, r) and aq + 1 (w, r).
-      const int ad = aq + 1;
-      const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-      const bool out = !in;
-      int l0[5], l1[5];
-      xs_warp_limbs((xs_int)v0, l0);
-      xs_warp_limbs((xs_int)v1, l1);
-      const unsigned outw = __ballot_sync(0xffffffffu, out);
-      if (lane == 0) {
-#pragma unroll
-        for (int k = 0; k < 5; k++) {
-          s_limb[wid][k] = l0[k];
-          s_limb[wid][5 + k] = l1[k];
-        }
-        s_limb[wid][10] = outw != 0;
-      }
-      __syncthreads();  // also orders this CTA's published edge values before the release below
-      unsigned long long* const slot = slots + (it % PCG_SLOTS) * PCG_SLOT_U64;
-      if (wid == 0 && lane >= 1 && lane < PCG_SLOT_WORDS) {
-        long long S = 0;
-#pragma unroll
-        for (int w = 0; w < PCG_T / 32; w++) S += s_limb[w][lane];
-        red_add_u64(slot + lane * PCG_WORD_STRIDE, ((unsigned long long)S << 8) + 1ull);
-      } else if (threadIdx.x == 64) {
-        long long S = 0;
-#pragma unroll
-        for (int w = 0; w < PCG_T / 32; w++) S += s_limb[w][0];
-        red_release_add_u64(slot, ((unsigned long long)S << 8) + 1ull);
-      }
-      // Warp 0 polls: lanes 0-4 the (w, r) limb words 0-4, lanes 8-12 the
-      // (r, r) words 5-9, lane 16 word 10 (so that each total gathers in an
-      // 8-lane group).
-      const int pword = lane < 5 ? lane : (lane >= 8 && lane < 13) ? lane - 3 : lane == 16 ? 10 : -1;
-      unsigned long long wv0 = 0;
-      if (wid == 0 && pword >= 0)
-        wv0 = lane == 0 ? ld_acquire_u64(slot) : ld_relaxed_u64(slot + pword * PCG_WORD_STRIDE);
-      // Deferred update of the previous iteration (no other CTA needs p' or
-      // x), and the scalars the next step needs from the previous ones.
-#pragma unroll
-      for (int j = 0; j < NPT; j++)
-        if (kk[j] >= 0) {
-          p[j] = fma(be, p[j], r_old[j]);
-          x[j] = fma(alq, p[j], x[j]);
-        }
-      if (threadIdx.x == 32) {
-        const double ri = recip_nr(s_rr);
-        s_rrinv = ri;
-        s_g = s_eta * (ri * ri);
-      }
-      if (wid == 0) {
-        unsigned long long wv = 0;
-        int good = 1;
-        if (pword >= 0) {
-          long long spins = 0;
-          wv = wv0;
-          for (;;) {
-            if ((wv & 255ull) == (unsigned long long)nb) break;
-            if (++spins >= spin) {
-              atomicOr(a.flags, FLAG_TIMEOUT);
-              good = 0;
-              break;
-            }
-            wv = lane == 0 ? ld_acquire_u64(slot) : ld_relaxed_u64(slot + pword * PCG_WORD_STRIDE);
-          }
-        }
-        good = __all_sync(0xffffffffu, good);
-        if (blockIdx.x == 0 && pword >= 0)
-          slots[((it + PCG_SLOTS - 1) % PCG_SLOTS) * PCG_SLOT_U64 + pword * PCG_WORD_STRIDE] = 0ull;
-        const long long S = pword >= 0 ? (long long)(wv - (unsigned long long)nb) >> 8 : 0;
-        const long long outc = __shfl_sync(0xffffffffu, S, 16);
-        // Each 8-lane group sums its limbs shifted to their weights (a
-        // butterfly of 128-bit adds): lane 0 holds (w, r), lane 8 (r, r);
-        // both round their totals at once.
-        xs_int V = (lane & 7) < 5 && lane < 16 ? (xs_int)S << (26 * (lane & 7)) : (xs_int)0;
-#pragma unroll
-        for (int o = 4; o >= 1; o >>= 1) {
-          const uint64_t vlo = (uint64_t)(xs_uint)V, vhi = (uint64_t)((xs_uint)V >> 64);
-          const uint64_t olo = __shfl_xor_sync(0xffffffffu, vlo, o), ohi = __shfl_xor_sync(0xffffffffu, vhi, o);
-          V += (xs_int)(((xs_uint)ohi << 64) | olo);
-        }
-        const double d = xs_to_double(V, lane == 0 ? ad : aq);
-        const double d1 = __shfl_sync(0xffffffffu, d, 8);
-        if (lane == 0) {
-          dr = d;
-          rr = d1;
-          s_ok = good;
-          s_exact = outc != 0;
-        }
-      }
-      __syncthreads();
-      if (!s_ok) return;
-      exact = s_exact;
-    }
-    if (exact) {
-      // Block-anchored reduction: partials of this episode's parity, then
-      // the grid totals after the counter barrier.
-      XPartial* const Pc = P + (ep & 1) * nb;
-      xs_block_partial<NPT>(td, tq, sx, Pc + blockIdx.x);
-      if (threadIdx.x == 0) bar_arrive(a.bar);
-      target += nb;
-      if (it > 0 && !fused) {
-#pragma unroll
-        for (int j = 0; j < NPT; j++)
-          if (kk[j] >= 0) {
-            p[j] = fma(be, p[j], r_old[j]);
-            x[j] = fma(alq, p[j], x[j]);
-          }
-        if (threadIdx.x == 32) {
-          const double ri = recip_nr(s_rr);
-          s_rrinv = ri;
-          s_g = s_eta * (ri * ri);
-        }
-      }
-      if (!bar_wait(a.bar, a.flags, target, &s_ok, spin)) return;
-      if (threadIdx.x < 32) xs_grid_totals_w0(Pc, nb, &dr, &rr);
-      ep++;
-    }
-    // Halo inputs published before the barrier, loaded while thread 0 forms
-    // the scalars.
-    const double* const pr_c = cur ? a.work[2] : a.work[1];
-    const double* const pw_c = cur ? a.work[4] : a.work[3];
-    const double* const ps_c = cur ? a.work[6] : a.work[5];
-    double hr[PCG_HALO_SLOTS], hw[PCG_HALO_SLOTS], hsv[PCG_HALO_SLOTS];
-#pragma unroll
-    for (int j = 0; j < PCG_HALO_SLOTS; j++)
-      if (he[j] >= 0) {
-        hr[j] = __ldcg(&pr_c[he[j]]);
-        hw[j] = __ldcg(&pw_c[he[j]]);
-        hsv[j] = __ldcg(&ps_c[he[j]]);
-      }
-    if (threadIdx.x == 0) {
-      s_rr = rr;
-      s_done = xs_bits(rr) < a.tol_bits || it >= maxit;  // sqrt(r.r) < tol
-      double beta, eta_r;
-      if (it == 0) {
-        beta = 0;
-        eta_r = dr;
-      } else {
-        beta = rr * s_rrinv;
-        eta_r = fma(-(rr * rr), s_g, dr);
-      }
-      s_eta = eta_r;
-      s_alpha = div_nr(rr, eta_r);
-      s_beta = beta;
-      s_aq = xs_exponent(rr) + PCG_ANCHOR_HEADROOM;
-    }
-    __syncthreads();
-    if (s_done) break;
-    const double al = s_alpha;
-    be = s_beta;
-    alq = -0.25 * al;
-    aq = s_aq;
-#pragma unroll
-    for (int j = 0; j < NPT; j++)
-      if (kk[j] >= 0) {
-        r_old[j] = r[j];
-        s[j] = fma(be, s[j], w[j]);
-        r[j] = fma(-al, s[j], r[j]);
-        sr[si[j]] = r[j];
-      }
-#pragma unroll
-    for (int j = 0; j < PCG_HALO_SLOTS; j++)
-      if (he[j] >= 0) sr[hs[j]] = fma(-al, fma(be, hsv[j], hw[j]), hr[j]);
-    __syncthreads();
-    double* const pr_n = cur ? a.work[1] : a.work[2];
-    double* const pw_n = cur ? a.work[3] : a.work[4];
-    double* const ps_n = cur ? a.work[5] : a.work[6];
-    v0 = v1 = 0;
-    in = true;
-#pragma unroll
-    for (int j = 0; j < NPT; j++)
-      if (kk[j] >= 0) {
-        const double* c = sr + si[j];
-        w[j] = fma(-0.25, (c[-ldu] + c[-1]) + (c[1] + c[ldu]), r[j]);
-        td[j] = w[j] * r[j];
-        tq[j] = r[j] * r[j];
-        if (fused) {
-          in &= xs_add_anchored<false>(v0, td[j], aq + 1);
-          in &= xs_add_anchored<true>(v1, tq[j], aq);
-        }
-        if (pe0[j] >= 0) {
-          pr_n[pe0[j]] = r[j];
-          pw_n[pe0[j]] = w[j];
-          ps_n[pe0[j]] = s[j];
-        }
-        if (pe1[j] >= 0) {
-          pr_n[pe1[j]] = r[j];
-          pw_n[pe1[j]] = w[j];
-          ps_n[pe1[j]] = s[j];
-        }
-      }
-    it++;
-  }
-  // domain.error = |A x - b| / n (src/field.cpp:258-259), n = nx ny.  With
-  // PERIODIC the same reduction also totals x, whose mean is then removed
-  // (the zero-mean gauge; the error is that of x before the shift).
-#pragma unroll
-  for (int j = 0; j < NPT; j++)
-    if (kk[j] >= 0) a.phi[kk[j]] = x[j];
-  __syncthreads();
-  if (threadIdx.x == 0) bar_arrive(a.bar);
-  target += nb;
-  if (!bar_wait(a.bar, a.flags, target, &s_ok, spin)) return;
-  const bool gauge = lat.mode == EPIC_POISSON_PERIODIC;
-#pragma unroll
-  for (int j = 0; j < NPT; j++) {
-    td[j] = tq[j] = 0.0;
-    if (kk[j] >= 0) {
-      const int q = threadIdx.x + PCG_T * j, lr = q / tc, lc = q - lr * tc;
-      const int row = r0 + lr, col = c0 + lc;
-      const int up = lattice_wrap(row - 1, R, lat.wrap_r), dn = lattice_wrap(row + 1, R, lat.wrap_r);
-      const int lf = lattice_wrap(col - 1, C, lat.wrap_c), rt = lattice_wrap(col + 1, C, lat.wrap_c);
-      double sum = 0;
-      if (up >= 0) sum += __ldcg(&a.phi[lattice_node(lat, up, col)]);
-      if (lf >= 0) sum += __ldcg(&a.phi[lattice_node(lat, row, lf)]);
-      sum = fma(-4.0, x[j], sum);
-      if (rt >= 0) sum += __ldcg(&a.phi[lattice_node(lat, row, rt)]);
-      if (dn >= 0) sum += __ldcg(&a.phi[lattice_node(lat, dn, col)]);
-      const double e = sum - (rhs(kk[j]) - bmean);
-      td[j] = e * e;
-      if (gauge) tq[j] = x[j];
-    }
-  }
-  XPartial* const Pe = P + (ep & 1) * nb;
-  xs_block_partial<NPT>(td, tq, sx, Pe + blockIdx.x);
-  if (threadIdx.x == 0) bar_arrive(a.bar);
-  target += nb;
-  if (!bar_wait(a.bar, a.flags, target, &s_ok, spin)) return;
-  if ((gauge || blockIdx.x == 0) && threadIdx.x < 32) {
-    double e2 = 0, xsum = 0;
-    xs_grid_totals_w0(Pe, nb, &e2, &xsum);
-    if (threadIdx.x == 0) {
-      s_mean = xsum / (double)n;
-      if (blockIdx.x == 0) {
-        a.info->iterations = it;
-        a.info->converged = it < maxit;
-        a.info->error = sqrt(e2) / (a.g.nx * a.g.ny);
-        atomicAdd(a.iter_total, (unsigned long long)it);
-      }
-    }
-  }
-  if (gauge) {
-    __syncthreads();
-    const double xm = s_mean;
-#pragma unroll
-    for (int j = 0; j < NPT; j++)
-      if (kk[j] >= 0) a.phi[kk[j]] = x[j] - xm;
-  }
-}
-
-// Tile shape for at most max_blocks CTAs: the fewest FP64 operations on the
-// busiest CTA (11 per owned node, 3 per halo node), ties to fewer CTAs.
-// Returns false when no tile fits PCG_T * 8 owned nodes and a halo ring of
-// PCG_T * PCG_HALO_SLOTS nodes (then the global-memory k_pcg runs).
-static bool pcg_tiling(int R, int C, int wrap_r, int wrap_c, int max_blocks, PcgTiling* out) {
-  long long best = -1;
-  PcgTiling b{};
-  for (int tcb = 1; tcb <= C && tcb <= max_blocks; tcb++) {
-    const int tc = (C + tcb - 1) / tcb;
-    const int ncb = (C + tc - 1) / tc;
-    const int rb_max = max_blocks / ncb;
-    if (rb_max < 1) continue;
-    const int tr = (R + rb_max - 1) / rb_max;
-    const int nrb = (R + tr - 1) / tr;
-    const long long nodes = (long long)tr * tc;
-    if (nodes > PCG_T * 8 || 2LL * (tr + tc) > PCG_T * PCG_HALO_SLOTS) continue;
-    if (ncb * nrb > PCG_MAX_BLOCKS) continue;
-    // Where the lattice wraps, the last tile's valid extent has a neighbour
-    // beyond both of its sides and must span two nodes (so that its first
-    // and last rows / columns are different nodes).
-    if ((wrap_r && R - (nrb - 1) * tr < 2) || (wrap_c && C - (ncb - 1) * tc < 2)) continue;
-    // The edge buffers (2 (tr + tc) slots per tile) live in node-sized vectors.
-    if (tr < 2 || tc < 2 || (long long)ncb * nrb * 2 * (tr + tc) > (long long)R * C) continue;
-    const long long cost = 11 * nodes + 3 * 2LL * (tr + tc);
-    const int blocks = ncb * nrb;
-    if (best < 0 || cost < best || (cost == best && blocks < b.blocks)) {
-      best = cost;
-      b.tr = tr;
-      b.tc = tc;
-      b.tiles_c = ncb;
-      b.blocks = blocks;
-      const int npt = (int)((nodes + PCG_T - 1) / PCG_T);
-      b.npt = npt <= 1 ? 1 : npt <= 2 ? 2 : npt <= 4 ? 4 : 8;
-    }
-  }
-  if (best < 0) return false;
-  *out = b;
-  return true;
-}
-
 int pcg_default_blocks(long long nodes, int sms) {
-  // One CTA per SM at most (FP64 throughput is per SM; more CTAs only add
-  // barrier arrivals), and no fewer than ~384 nodes per CTA on small grids.
-  long long want = (nodes + 383) / 384;
+  // One CTA per SM at most: FP64 throughput is per SM, more CTAs only add
+  // words to exchange.
+  long long want = (nodes + 63) / 64;
   return (int)std::max(1LL, std::min<long long>(want, std::min(solver_max_blocks(), sms)));
 }
 
-// Launches the tiled solve if all its CTAs can be resident at once (the
-// cooperative-launch condition); returns false otherwise.
-template <int NPT>
-static bool launch_tiled(cudaStream_t st, const SolverArgs& a, const PcgTiling& t) {
-  const int smem = (t.tr + 2) * (t.tc + 2) * (int)sizeof(double);
-  int dev = 0, sms = 0, per_sm = 0;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_pcg_tiled<NPT>, PCG_T, smem);
-  if (t.blocks > per_sm * sms) return false;
-  SolverArgs args = a;
-  PcgTiling tl = t;
-  void* params[] = {&args, &tl};
-  cudaLaunchCooperativeKernel((const void*)k_pcg_tiled<NPT>, dim3(t.blocks), dim3(PCG_T), params, smem, st);
-  return true;
-}
-
-void launch_pcg(cudaStream_t st, const SolverArgs& a_in, int blocks) {
+int launch_pcg(cudaStream_t st, const SolverArgs& a_in, int blocks) {
   cudaMemsetAsync(a_in.bar, 0, 2 * sizeof(unsigned int), st);
   SolverArgs a = a_in;
   a.spin = spin_limit();
-  const Lattice lat = make_lattice(a.g.nx, a.g.ny, a.poisson_bc);
-  PcgTiling t;
-  if (pcg_tiling(lat.R, lat.C, lat.wrap_r, lat.wrap_c, blocks, &t)) {
-    SolverArgs at = a;
-    at.tol_bits = xs_bits(xs_sqrt_threshold(a.tol));
-    bool ok;
-    switch (t.npt) {
-      case 1: ok = launch_tiled<1>(st, at, t); break;
-      case 2: ok = launch_tiled<2>(st, at, t); break;
-      case 4: ok = launch_tiled<4>(st, at, t); break;
-      default: ok = launch_tiled<8>(st, at, t); break;
-    }
-    if (ok) {
-      if (a.poisson_bc != EPIC_POISSON_DIRICHLET) launch_fill_poisson_nodes(st, a.g, a.poisson_bc, a.phi);
-      return;
-    }
-  }
+  if (launch_pcg_modes(st, a, blocks)) return 1;
   SolverArgs args = a;
   void* params[] = {&args};
   cudaLaunchCooperativeKernel((const void*)k_pcg, dim3(blocks), dim3(256), params, 0, st);
-  if (a.poisson_bc != EPIC_POISSON_DIRICHLET) launch_fill_poisson_nodes(st, a.g, a.poisson_bc, a.phi);
+  if (a.poisson_bc == EPIC_POISSON_DIRICHLET) return 1;
+  launch_fill_poisson_nodes(st, a.g, a.poisson_bc, a.phi);
+  return 2;
 }
 
 __global__ void k_fill_poisson_nodes(Geom g, int mode, double* phi) {

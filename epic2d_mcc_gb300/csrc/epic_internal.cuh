@@ -419,7 +419,8 @@ void launch_sor_lex(cudaStream_t st, const SolverArgs& a);
 void launch_gsfluid(cudaStream_t st, const SolverArgs& a, double* rho);
 void launch_nrpcg(cudaStream_t st, const SolverArgs& a);
 void launch_sor_redblack(cudaStream_t st, const SolverArgs& a, int blocks);
-void launch_pcg(cudaStream_t st, const SolverArgs& a, int blocks);
+int launch_pcg(cudaStream_t st, const SolverArgs& a, int blocks);  // kernels launched
+bool launch_pcg_modes(cudaStream_t st, const SolverArgs& a, int max_blocks);  // epic_pcg.cu
 int solver_max_blocks();
 // CTA budget of a PCG solve on `nodes` unknowns (shared by every entry point
 // that runs it, so they all produce the same iterates).
