@@ -132,41 +132,6 @@ __device__ double block_sum_1024(double v, double* sm) {
   return t;
 }
 
-// ---- exact dot-product reductions (integer pipe, epic_xsum.cuh) ----
-// Exact sum of term(q), q in [0, count), over the block (each thread takes a
-// strided share), anchored on the largest exponent and rounded once
-// (epic_xsum.cuh); valid in every thread.
-template <class F>
-__device__ double block_exact_sum(int count, const F& term, double* red) {
-  __shared__ int s_e[32];
-  __shared__ unsigned long long s_v[32][2];
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  int e = 0;
-  for (int q = threadIdx.x; q < count; q += blockDim.x) e = max(e, xs_exponent(term(q)));
-  e = (int)__reduce_max_sync(0xffffffffu, (unsigned)e);
-  if (lane == 0) s_e[wid] = e;
-  __syncthreads();
-  int A = 0;
-  for (int w = 0; w < nw; w++) A = max(A, s_e[w]);
-  xs_int v = 0;
-  for (int q = threadIdx.x; q < count; q += blockDim.x) v += xs_from_double(term(q), A);
-  v = xs_warp_sum(v);
-  if (lane == 0) {
-    s_v[wid][0] = (unsigned long long)(xs_uint)v;
-    s_v[wid][1] = (unsigned long long)((xs_uint)v >> 64);
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    xs_uint tot = 0;
-    for (int w = 0; w < nw; w++) tot += ((xs_uint)s_v[w][1] << 64) | s_v[w][0];
-    red[33] = xs_to_double((xs_int)tot, A);
-  }
-  __syncthreads();
-  const double r = red[33];
-  __syncthreads();
-  return r;
-}
-
 // The unknowns of gssolver: the interior i in [1, nx-2], j in [1, ny-2]
 // (the reference), or an extension lattice (EPIC_POISSON_*): i from i0 = 0
 // (PERIODIC) or 1 (DIRICHLET_X) to nx-2, j in [0, ny-2], with wrapped
@@ -741,7 +706,8 @@ void launch_sor_lex(cudaStream_t st, const SolverArgs& a) {
   const int use_smem = 2 * bytes <= SOR_SMEM_MAX ? 2 : bytes <= SOR_SMEM_MAX ? 1 : 0;
   const size_t smem = use_smem * bytes;
   if (a.poisson_bc != EPIC_POISSON_DIRICHLET) {
-    const bool cl = sor_unit(a) ? launch_sor_cluster<false, true, true>(st, a)
+    const bool cl = launch_sor_rows(st, a) ? true
+                    : sor_unit(a) ? launch_sor_cluster<false, true, true>(st, a)
                                 : launch_sor_cluster<false, false, true>(st, a);
     if (!cl) {
       if (sor_unit(a)) k_sor_lex<false, true, true><<<1, SOR_THREADS, smem, st>>>(a, use_smem);

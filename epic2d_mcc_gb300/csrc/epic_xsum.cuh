@@ -164,6 +164,40 @@ __device__ __forceinline__ xs_int xs_warp_sum(xs_int v) {
                     ((xs_uint)(unsigned)l1 << 26) + (xs_uint)(unsigned)l0;
   return (xs_int)s;
 }
+
+// Exact sum of term(q), q in [0, count), over the block (each thread takes a
+// strided share), anchored on the largest exponent and rounded once
+// (epic_xsum.cuh); valid in every thread.
+template <class F>
+__device__ double block_exact_sum(int count, const F& term, double* red) {
+  __shared__ int s_e[32];
+  __shared__ unsigned long long s_v[32][2];
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  int e = 0;
+  for (int q = threadIdx.x; q < count; q += blockDim.x) e = max(e, xs_exponent(term(q)));
+  e = (int)__reduce_max_sync(0xffffffffu, (unsigned)e);
+  if (lane == 0) s_e[wid] = e;
+  __syncthreads();
+  int A = 0;
+  for (int w = 0; w < nw; w++) A = max(A, s_e[w]);
+  xs_int v = 0;
+  for (int q = threadIdx.x; q < count; q += blockDim.x) v += xs_from_double(term(q), A);
+  v = xs_warp_sum(v);
+  if (lane == 0) {
+    s_v[wid][0] = (unsigned long long)(xs_uint)v;
+    s_v[wid][1] = (unsigned long long)((xs_uint)v >> 64);
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    xs_uint tot = 0;
+    for (int w = 0; w < nw; w++) tot += ((xs_uint)s_v[w][1] << 64) | s_v[w][0];
+    red[33] = xs_to_double((xs_int)tot, A);
+  }
+  __syncthreads();
+  const double r = red[33];
+  __syncthreads();
+  return r;
+}
 #endif
 
 }  // namespace epic
