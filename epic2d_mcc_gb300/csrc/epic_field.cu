@@ -716,6 +716,7 @@ void launch_sor_lex(cudaStream_t st, const SolverArgs& a) {
     launch_fill_poisson_nodes(st, a.g, a.poisson_bc, a.phi);
     return;
   }
+  if (launch_sor_stream(st, a, false)) return;
   if (sor_unit(a) ? launch_sor_cluster<false, true, false>(st, a) : launch_sor_cluster<false, false, false>(st, a))
     return;
   if (sor_unit(a)) k_sor_lex<false, true, false><<<1, SOR_THREADS, smem, st>>>(a, use_smem);
@@ -739,6 +740,7 @@ __global__ void k_gsfluid_edges(Geom g, double* rho, double top) {
 
 void launch_gsfluid(cudaStream_t st, const SolverArgs& a, double* rho) {
   k_gsfluid_edges<<<1, 256, 0, st>>>(a.g, rho, 10000 * (QE / (K_B * (QE / K_B))));
+  if (launch_sor_stream(st, a, true)) return;
   const size_t bytes = (size_t)a.g.nx * a.g.ny * sizeof(double);
   const int use_smem = bytes <= SOR_SMEM_MAX;
   if (sor_unit(a) ? launch_sor_cluster<true, true, false>(st, a) : launch_sor_cluster<true, false, false>(st, a))

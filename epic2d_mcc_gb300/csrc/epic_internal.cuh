@@ -415,6 +415,7 @@ void init_field_kernels();  // one-time kernel attributes (called by epic_create
 void set_last_error(const char* msg);  // the message epic_last_error() returns on this thread
 void launch_sor_lex(cudaStream_t st, const SolverArgs& a);
 bool launch_sor_rows(cudaStream_t st, const SolverArgs& a);  // epic_sor.cu
+bool launch_sor_stream(cudaStream_t st, const SolverArgs& a, bool fluid);
 // Boltzmann-electron solvers: gsfluidsolver ("gshybrid"; writes rho's edge
 // values, as the reference does) and nrpcgsolver ("hybrid").
 void launch_gsfluid(cudaStream_t st, const SolverArgs& a, double* rho);

@@ -215,7 +215,7 @@ __device__ __forceinline__ void pm_store_cluster(unsigned addr, unsigned long lo
 }
 __device__ __forceinline__ unsigned long long pm_load_cta(const unsigned long long* p) {
   unsigned long long v;
-  asm volatile("ld.relaxed.cluster.shared::cta.u64 %0, [%1];"
+  asm volatile("ld.volatile.shared::cta.u64 %0, [%1];"
                : "=l"(v)
                : "r"((unsigned)__cvta_generic_to_shared(p))
                : "memory");
