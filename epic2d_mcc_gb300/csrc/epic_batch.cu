@@ -571,15 +571,15 @@ __global__ void k_batch_spec_check(BatchSpec b, int nruns, int final_pass) {
 
 // One of the four products of a refinement stage for every (run, tile) of
 // the schedule: 0 t1 = Q_R t0; 1 t0 = (t1 Q_C) o D; 2 t1 = Q_R t0; 3 phi += t1 Q_C.
-// TILE 16 or 32: spec_gemm_tile; 64: the register-blocked spec_gemm_tile64
+// TILE 16: spec_gemm_panel16; 32: spec_gemm_tile; 64: the register-blocked spec_gemm_tile64
 // (the same k order, so the same results).
 template <int PROD, int TILE>
 __global__ void __launch_bounds__(256) k_batch_spec_gemm(BatchSpec b, const int4* __restrict__ sched) {
   const int4 e = sched[blockIdx.x];  // (run, tile row, tile col)
   if (b.state[4 * e.x]) return;
-  __shared__ float As[TILE == 64 ? 1 : 32][33];
-  __shared__ float Bs[TILE == 64 ? 1 : 32][33];
-  __shared__ __align__(16) SpecGemmSmem sg[TILE == 64 ? 1 : 1];
+  __shared__ float As[TILE == 32 ? 32 : 1][33];
+  __shared__ float Bs[TILE == 32 ? 32 : 1][33];
+  __shared__ __align__(16) unsigned char s_ops[TILE == 64 ? sizeof(SpecGemmSmem) : TILE == 16 ? sizeof(SpecPanel) : 16];
   const BRun& r = b.runs[e.x];
   const SpecLattice L = run_lattice(b, e.x);
   float* t0 = b.t0 + r.lat_off;
@@ -587,9 +587,15 @@ __global__ void __launch_bounds__(256) k_batch_spec_gemm(BatchSpec b, const int4
   const float* QR = b.Q + r.qR_off;
   const float* QC = b.Q + r.qC_off;
   if constexpr (TILE == 64) {
-    if (PROD == 0 || PROD == 2) spec_gemm_tile64<0>(r.R, r.C, r.R, QR, t0, t1, nullptr, &L, e.y, e.z, sg[0]);
-    else if (PROD == 1) spec_gemm_tile64<1>(r.R, r.C, r.C, t1, QC, t0, b.D + r.lat_off, &L, e.y, e.z, sg[0]);
-    else spec_gemm_tile64<2>(r.R, r.C, r.C, t1, QC, nullptr, nullptr, &L, e.y, e.z, sg[0]);
+    SpecGemmSmem& sg = *reinterpret_cast<SpecGemmSmem*>(s_ops);
+    if (PROD == 0 || PROD == 2) spec_gemm_tile64<0>(r.R, r.C, r.R, QR, t0, t1, nullptr, &L, e.y, e.z, sg);
+    else if (PROD == 1) spec_gemm_tile64<1>(r.R, r.C, r.C, t1, QC, t0, b.D + r.lat_off, &L, e.y, e.z, sg);
+    else spec_gemm_tile64<2>(r.R, r.C, r.C, t1, QC, nullptr, nullptr, &L, e.y, e.z, sg);
+  } else if constexpr (TILE == 16) {
+    SpecPanel& sp = *reinterpret_cast<SpecPanel*>(s_ops);
+    if (PROD == 0 || PROD == 2) spec_gemm_panel16<0>(r.R, r.C, r.R, QR, t0, t1, nullptr, &L, e.y, e.z, sp);
+    else if (PROD == 1) spec_gemm_panel16<1>(r.R, r.C, r.C, t1, QC, t0, b.D + r.lat_off, &L, e.y, e.z, sp);
+    else spec_gemm_panel16<2>(r.R, r.C, r.C, t1, QC, nullptr, nullptr, &L, e.y, e.z, sp);
   } else {
     if (PROD == 0 || PROD == 2)
       spec_gemm_tile<0, TILE>(r.R, r.C, r.R, QR, t0, t1, nullptr, &L, e.y, e.z, As, Bs);

@@ -166,9 +166,10 @@ __global__ void __launch_bounds__(256) k_spec_solve(SpecLattice L, const float* 
                                                     float* t1, int stages, unsigned int* bar, int* flags,
                                                     long long spin, SpecFFT F) {
   extern __shared__ float2 fbuf[];
-  __shared__ __align__(16) float As[TILE == 64 || TILE == 0 ? 1 : 32][33];
-  __shared__ float Bs[TILE == 64 || TILE == 0 ? 1 : 32][33];
-  __shared__ __align__(16) SpecGemmSmem sg[TILE == 64 ? 1 : 0 + 1];
+  // operands of a product's tile
+  __shared__ __align__(16) float As[TILE == 32 ? 32 : 1][33];
+  __shared__ float Bs[TILE == 32 ? 32 : 1][33];
+  __shared__ __align__(16) unsigned char s_ops[TILE == 64 ? sizeof(SpecGemmSmem) : TILE == 16 ? sizeof(SpecPanel) : 16];
   __shared__ double sm8[8];
   __shared__ double s_mean, s_sum;
   __shared__ int s_stop;
@@ -216,11 +217,13 @@ __global__ void __launch_bounds__(256) k_spec_solve(SpecLattice L, const float* 
     if (s_stop) break;
 #define SPEC_PASS(EPI, K_, A_, B_, C_, D_)                                                                    \
   for (int t = blockIdx.x; t < ntiles; t += gridDim.x) {                                                       \
-    if (TILE == 64)                                                                                          \
-      spec_gemm_tile64<EPI>(R, C, K_, A_, B_, C_, D_, &L, t / tiles_c, t - (t / tiles_c) * tiles_c, sg[0]);  \
-    else                                                                                                     \
-      spec_gemm_tile<EPI, TILE == 64 ? 32 : TILE>(R, C, K_, A_, B_, C_, D_, &L, t / tiles_c,                 \
-                                                  t - (t / tiles_c) * tiles_c, As, Bs);                      \
+    const int tr = t / tiles_c, tc = t - tr * tiles_c;                                                         \
+    if constexpr (TILE == 64)                                                                                  \
+      spec_gemm_tile64<EPI>(R, C, K_, A_, B_, C_, D_, &L, tr, tc, *reinterpret_cast<SpecGemmSmem*>(s_ops));    \
+    else if constexpr (TILE == 16)                                                                             \
+      spec_gemm_panel16<EPI>(R, C, K_, A_, B_, C_, D_, &L, tr, tc, *reinterpret_cast<SpecPanel*>(s_ops));      \
+    else                                                                                                       \
+      spec_gemm_tile<EPI, 32>(R, C, K_, A_, B_, C_, D_, &L, tr, tc, As, Bs);                                   \
   }                                                                                                          \
   if (!spec_grid_sync(bar, flags, spin)) return;
 #define SPEC_FFT(EPI, DIR, IN_, OUT_, D_)                                                         \

@@ -214,8 +214,8 @@ __device__ __forceinline__ void spec_add_phi(const SpecLattice* L, int N, int r,
   *ph = __ldcg(ph) + (double)v;
 }
 
-// One TILE x TILE output tile of C = A B (M x K by K x N, row-major FP32) at
-// tile (tr, tc), 256 threads.  EPI 0: store; 1: store C o D; 2: add to phi
+// One 32 x 32 output tile of C = A B (M x K by K x N, row-major FP32) at tile
+// (tr, tc), 256 threads.  EPI 0: store; 1: store C o D; 2: add to phi
 // (FP64) at the node of lattice entry (r, c).
 template <int EPI, int TILE>
 __device__ __forceinline__ void spec_gemm_tile(int M, int N, int K, const float* __restrict__ A,
@@ -256,6 +256,62 @@ __device__ __forceinline__ void spec_gemm_tile(int M, int N, int K, const float*
       else if (EPI == 1) Cm[r * N + c] = acc[a][b] * D[r * N + c];
       else spec_add_phi(L, N, r, c, acc[a][b]);
     }
+}
+
+// The same for 16 x 16 tiles: whole panels of SP_K steps of k in shared memory,
+// both along k, so that a thread takes four steps per 16-byte load.  A product
+// of a lattice with 16-wide tiles is bound by the latency of its loads (its
+// operands lie in L2) and by the shared-memory loads: tile-wide steps of k, a
+// barrier on each side, paid the first 17 times at 257 x 257 (~10 us a product),
+// a panel pays it once (~4 us).
+constexpr int SP_K = 256, SP_LD = SP_K + 4;
+struct SpecPanel {
+  float A[16][SP_LD], B[16][SP_LD];  // B transposed
+};
+template <int EPI>
+__device__ __forceinline__ void spec_gemm_panel16(int M, int N, int K, const float* __restrict__ A,
+                                                  const float* __restrict__ B, float* __restrict__ Cm,
+                                                  const float* __restrict__ D, const SpecLattice* L, int tr, int tc,
+                                                  SpecPanel& sm) {
+  const int lo = threadIdx.x & 15, hi = threadIdx.x >> 4;
+  const int row0 = tr * 16, col0 = tc * 16;
+  const bool arow = row0 + hi < M, bcol = col0 + lo < N;
+  float acc = 0.f;
+  for (int k0 = 0; k0 < K; k0 += SP_K) {
+    const int kn = min(SP_K, K - k0), kp = (kn + 3) & ~3;  // zeros up to whole quads
+    const float* const a = A + (size_t)(row0 + hi) * K + k0 + lo;   // row hi, k lo + 16 u
+    const float* const b = B + (size_t)(k0 + hi) * N + col0 + lo;   // k hi + 16 u, column lo
+    for (int u0 = 0; u0 < kp; u0 += 128) {
+      float va[8], vb[8];
+#pragma unroll
+      for (int u = 0; u < 8; u++) {
+        const int ka = u0 + 16 * u + lo, kb = u0 + 16 * u + hi;
+        va[u] = arow && ka < kn ? __ldcg(a + u0 + 16 * u) : 0.f;
+        vb[u] = bcol && kb < kn ? __ldcg(b + (size_t)(u0 + 16 * u) * N) : 0.f;
+      }
+#pragma unroll
+      for (int u = 0; u < 8; u++) {
+        sm.A[hi][u0 + 16 * u + lo] = va[u];
+        sm.B[lo][u0 + 16 * u + hi] = vb[u];
+      }
+    }
+    __syncthreads();
+#pragma unroll 4
+    for (int k = 0; k < kp; k += 4) {
+      const float4 x = *reinterpret_cast<const float4*>(&sm.A[hi][k]);
+      const float4 y = *reinterpret_cast<const float4*>(&sm.B[lo][k]);
+      acc = fmaf(x.x, y.x, acc);
+      acc = fmaf(x.y, y.y, acc);
+      acc = fmaf(x.z, y.z, acc);
+      acc = fmaf(x.w, y.w, acc);
+    }
+    __syncthreads();
+  }
+  const int r = row0 + hi, c = col0 + lo;
+  if (r >= M || c >= N) return;
+  if (EPI == 0) Cm[r * N + c] = acc;
+  else if (EPI == 1) Cm[r * N + c] = acc * D[r * N + c];
+  else spec_add_phi(L, N, r, c, acc);
 }
 
 // A 64 x 64 output tile of C = A B for large lattices, 256 threads with 4 x 4
