@@ -178,14 +178,24 @@ constexpr int PM_WIDEN = 24;
 constexpr int PM_DELAY = 400;
 constexpr unsigned long long PM_OUT = (1ull << 62) - 1;
 
-__device__ __forceinline__ void pm_term(unsigned long long& acc, bool& bad, double x, int E) {
-  const unsigned long long b = xs_bits(x);  // x >= 0
-  const int eb = (int)(b >> 52);
-  const unsigned long long m = (b & 0xFFFFFFFFFFFFFull) | ((unsigned long long)(eb != 0) << 52);
-  const int s = PM_TOP + (eb ? eb : 1) - E;
-  const unsigned long long dn = (xs_shr(m, (unsigned)(-s - 1)) + 1) >> 1;
-  acc += s >= 0 ? m << (s & 15) : dn;
-  bad |= s > 8 || eb >= 2047 || (acc >> 61) != 0;
+// r^2 and L r^2 of a component, added to the sums.  From the significands: a
+// 64 x 64-bit high product takes ~40 cycles of the integer pipe, an FP64 product
+// holds the warp's quarter of the SM for 64 and its result would have to be
+// taken apart again (an iteration at 257 x 257: 1.89 us with FP64 products,
+// 1.82 us so; with 16 components a thread, 1024 x 1024: 7.0 against 6.0 us).
+// Cut at 2^-62 of the term, where an FP64 product is rounded at 2^-53.
+__device__ __forceinline__ void pm_terms(unsigned long long& v0, unsigned long long& v1, bool& b0, bool& b1, double r,
+                                         double L, int E0, int E1) {
+  const unsigned long long b = xs_bits(r), l = xs_bits(L);  // L >= 0
+  const int eb = (int)((b >> 52) & 0x7FF), el = (int)(l >> 52);
+  const unsigned long long m = eb ? (b << 11) | (1ull << 63) : 0ull;  // |r| = m 2^(eb - 1086); below the normal range: 0
+  const unsigned long long lm = el ? (l << 11) | (1ull << 63) : 0ull;
+  const unsigned long long p = __umul64hi(m, m), q = __umul64hi(p, lm);  // r^2 = p 2^(2 eb - 2108), L r^2 = q 2^(2 eb + el - 3130)
+  const int n0 = E0 + 1027 - 2 * eb, n1 = E1 + 2049 - 2 * eb - el;      // shifts to the anchors
+  v0 += (xs_shr(p, (unsigned)(n0 - 1)) + 1) >> 1;
+  v1 += (xs_shr(q, (unsigned)(n1 - 1)) + 1) >> 1;
+  b0 |= eb >= 2047 || (m && n0 < 3) || (v0 >> 61) != 0;
+  b1 |= (m && n1 < 3) || (v1 >> 61) != 0;
 }
 
 // Warp total of v <= 2^61 in every lane, saturated to PM_OUT from 2^61 on.
@@ -647,9 +657,7 @@ __global__ void __launch_bounds__(PM_ALL) k_pcg_modes(SolverArgs a, PcgModes t) 
       for (int j = 0; j < NPT; j++) {
         if (wid * 32 + PM_T * j < t.per) {
           if (!again) r[j] = fma(-al, q[j], r[j]);
-          const double rr = r[j] * r[j];
-          pm_term(v0, b0, rr, E[0]);
-          pm_term(v1, b1, L[j] * rr, E[1]);
+          pm_terms(v0, v1, b0, b1, r[j], L[j], E[0], E[1]);
         }
       }
       v0 = pm_warp_sum(b0 ? 1ull << 61 : v0);
