@@ -304,6 +304,14 @@ static bool fused_deposit(const epic_sim* s) {
   return s->mixed ? s->cfg.shape == EPIC_CIC : s->cfg.deposit_mode == EPIC_DEPOSIT_FIXED;
 }
 
+// A mixed state that never sorts keeps its particles in the order they came in
+// and deposits them through shared-memory node words; one that sorts merges
+// neighbours instead (deposit_warp_sorted), which for sorted particles sends
+// an order of magnitude fewer atomics.
+static bool deposit_in_bands(const epic_sim* s) {
+  return s->mixed && s->cfg.shape == EPIC_CIC && s->cfg.sort_every == 0 && deposit_bands_fit(s->g);
+}
+
 static void invalidate_acc(epic_sim* s) {
   for (auto& sp : s->sp) sp.acc_valid = false;
 }
@@ -313,7 +321,9 @@ epic_status do_deposit(epic_sim* s, int i) {
   epic_species_state& sp = s->sp[i];
   sp.acc_valid = true;
   CK(cudaMemsetAsync(sp.acc, 0, nnodes(s) * sizeof(unsigned long long), s->stream));
-  if (s->mixed && s->cfg.shape == EPIC_CIC)
+  if (deposit_in_bands(s))
+    launch_deposit_mixed_bands(s->stream, s->g, sp.mx, sp.d_n, sp.acc);
+  else if (s->mixed && s->cfg.shape == EPIC_CIC)
     launch_deposit_mixed_sorted(s->stream, s->g, sp.mx, sp.d_n, sp.acc, s->part_grid);
   else if (s->mixed)
     launch_deposit_mixed(s->stream, s->g, s->cfg.shape, sp.mx, sp.d_n, sp.acc, s->d_flags, s->part_grid);
@@ -466,7 +476,9 @@ epic_status do_push(epic_sim* s, int i, int sub_cycle, const SelectArgs* sel = n
     const CondSet cs{s->cond_nrect, s->cond_ncirc, s->d_cond_rect, s->d_cond_circ, s->d_cond_live};
     launch_push_mixed(s->stream, s->g, c.shape, c.bc, sp.mx, sp.d_n, s->ef32, (float)(qmK * dtsub),
                       (float)(cc * dtsub / c.dx), (float)(cc * dtsub / c.dy), s->d_flags, s->tile_status,
-                      s->tile_ctr, s->part_grid, dep ? sp.acc : nullptr, dep ? sel : nullptr, cond ? &cs : nullptr);
+                      s->tile_ctr, s->part_grid, dep ? sp.acc : nullptr, dep ? sel : nullptr, cond ? &cs : nullptr,
+                      dep && deposit_in_bands(s));
+    if (dep && deposit_in_bands(s)) s->launches += 1;
     sp.acc_valid = dep;
   } else {
     const bool dep = fused_deposit(s);

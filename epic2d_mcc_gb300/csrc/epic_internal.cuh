@@ -252,12 +252,16 @@ int resident_grid(K kernel, int threads) {
 // With dep_acc (CIC, periodic or reflective walls) every pushed particle is
 // also deposited at its new position into dep_acc (integer weights), and with
 // sel the electrons' MCC candidates are appended to sel->cand.  With cond,
-// particles that end inside a conductor are erased (compacting push).
+// particles that end inside a conductor are erased (compacting push).  bands:
+// the deposit is a launch of its own (launch_deposit_mixed_bands).
 void launch_push_mixed(cudaStream_t st, const Geom& g, int shape, int bc, const MixedSoA& p, long long* d_n,
                        const float2* ef, float qmK_dt, float cx, float cy, int* flags,
                        unsigned long long* tile_status, unsigned int* tile_ctr, int grid,
                        unsigned long long* dep_acc = nullptr, const SelectArgs* sel = nullptr,
-                       const CondSet* cond = nullptr);
+                       const CondSet* cond = nullptr, bool bands = false);
+bool deposit_bands_fit(const Geom& g);
+void launch_deposit_mixed_bands(cudaStream_t st, const Geom& g, const MixedSoA& p, const long long* d_n,
+                                unsigned long long* acc);
 void launch_deposit_mixed_range(cudaStream_t st, const Geom& g, const MixedSoA& p, const long long* d_from,
                                 const long long* d_n, unsigned long long* acc, int grid);
 void launch_rewind_mixed(cudaStream_t st, const Geom& g, int shape, const MixedSoA& p, const long long* d_n,

@@ -11,6 +11,8 @@
 // FP64 oracle within stated tolerances, not bit for bit.
 #include <cuda_runtime.h>
 
+#include <algorithm>
+
 #include "epic_device.cuh"
 #include "epic_internal.cuh"
 #include "epic_mixed.cuh"
@@ -127,6 +129,115 @@ void launch_deposit_mixed_range(cudaStream_t st, const Geom& g, const MixedSoA& 
   k_deposit_mixed_range<<<grid, PART_THREADS, 0, st>>>(g, p, d_from, d_n, acc);
 }
 
+// CIC deposit of particles in no particular order (a state that never sorts).
+//
+// Sent straight to the grid, such particles are four 64-bit atomics each at
+// random addresses, and the L2's atomic units bound the pass; on small grids
+// equal addresses queue up as well.  Here a CTA owns a band of rows, holds its
+// node words in shared memory, goes through its slice of all particles, keeps
+// those of its band, and adds the words to the grid once at the end.  Bands
+// are as few as 220 KB a CTA allow: each particle is looked at once per band,
+// and only reading it (12 bytes, from L2 after the first band) is repeated.
+//
+// A word is two 32-bit halves, the low one added with the old value returned,
+// which tells the carry: shared memory has no 64-bit add, and its emulation as
+// a compare-and-swap loop took 2 to 3.5 times as long (8M particles on 64 x 64
+// cells, push and deposit: 205 us with it, 142 so, 582 by atomics on the grid;
+// 8 x 8: 436, 123, 1370; 256 x 256, three bands: 279, 222, 311).  What bounds
+// it are the eight shared-memory atomics of a particle.  Integer sums: the
+// order does not matter, and the result equals the other deposits'.
+constexpr int DT_THREADS = 1024;
+constexpr int DT_PER_THREAD = 8;  // consecutive particles a thread, loaded as vectors
+constexpr int DT_CHUNK = DT_THREADS * DT_PER_THREAD;
+constexpr int DT_MAX_SMEM = 220 * 1024;
+
+__device__ __forceinline__ void dt_add(unsigned* lo, unsigned* hi, int k, unsigned long long w) {
+  const unsigned l = (unsigned)w, old = atomicAdd(lo + k, l);
+  atomicAdd(hi + k, (unsigned)(w >> 32) + (old + l < l));
+}
+
+// Band b: cell rows [b rows, (b + 1) rows), node rows one more.
+__global__ void __launch_bounds__(DT_THREADS, 1) k_deposit_mixed_bands(Geom g, MixedSoA p,
+                                                                       const long long* __restrict__ d_n,
+                                                                       unsigned long long* __restrict__ acc, int bands,
+                                                                       int rows) {
+  extern __shared__ unsigned dt_words[];
+  constexpr int P = DT_PER_THREAD;
+  constexpr unsigned S = 1u << MIXED_OFFSET_BITS;
+  const float fS = (float)S;
+  const long long n = *d_n;
+  const int band = blockIdx.x % bands, slice = blockIdx.x / bands, slices = gridDim.x / bands;
+  const int r0 = band * rows, nr = min(rows, g.nx - 1 - r0);
+  const int c0 = r0 * g.ny, span = nr * g.ny, words = span + g.ny;
+  if ((long long)slice * DT_CHUNK >= n) return;
+  unsigned* const lo = dt_words;
+  unsigned* const hi = dt_words + words;
+  for (int k = threadIdx.x; k < 2 * words; k += DT_THREADS) dt_words[k] = 0;
+  __syncthreads();
+  for (long long chunk = (long long)slice * DT_CHUNK; chunk < n; chunk += (long long)slices * DT_CHUNK) {
+    const long long q0 = chunk + (long long)threadIdx.x * P;
+    int c[P];
+    float ox[P], oy[P];
+    if (q0 + P <= n) {
+#pragma unroll
+      for (int h = 0; h < P / 4; h++) {
+        const int4 cc = __ldg(reinterpret_cast<const int4*>(p.cell + q0) + h);
+        const float4 xx = __ldg(reinterpret_cast<const float4*>(p.ox + q0) + h);
+        const float4 yy = __ldg(reinterpret_cast<const float4*>(p.oy + q0) + h);
+        c[4 * h] = cc.x; c[4 * h + 1] = cc.y; c[4 * h + 2] = cc.z; c[4 * h + 3] = cc.w;
+        ox[4 * h] = xx.x; ox[4 * h + 1] = xx.y; ox[4 * h + 2] = xx.z; ox[4 * h + 3] = xx.w;
+        oy[4 * h] = yy.x; oy[4 * h + 1] = yy.y; oy[4 * h + 2] = yy.z; oy[4 * h + 3] = yy.w;
+      }
+    } else {
+#pragma unroll
+      for (int k = 0; k < P; k++) {
+        const long long q = q0 + k;
+        c[k] = q < n ? __ldg(&p.cell[q]) : -1;
+        ox[k] = q < n ? __ldg(&p.ox[q]) : 0.f;
+        oy[k] = q < n ? __ldg(&p.oy[q]) : 0.f;
+      }
+    }
+#pragma unroll
+    for (int k = 0; k < P; k++) {
+      const int m = c[k] - c0;
+      if ((unsigned)m < (unsigned)span) {
+        const unsigned a = (unsigned)(int)(ox[k] * fS), b = (unsigned)(int)(oy[k] * fS);
+        dt_add(lo, hi, m, (unsigned long long)(S - a) * (S - b));
+        dt_add(lo, hi, m + g.ny, (unsigned long long)a * (S - b));
+        dt_add(lo, hi, m + 1, (unsigned long long)(S - a) * b);
+        dt_add(lo, hi, m + g.ny + 1, (unsigned long long)a * b);
+      }
+    }
+  }
+  __syncthreads();
+  for (int k = threadIdx.x; k < words; k += DT_THREADS) {
+    const unsigned long long w = (unsigned long long)hi[k] << 32 | lo[k];
+    if (w) atomicAdd(acc + c0 + k, w);
+  }
+}
+
+// Grids of up to eight bands' words (475 x 475 nodes) whose rows are short
+// enough that a band has several.  Measured over whole steps: 400 x 400 cells
+// (six bands) 1.06 to 1.1 times as fast as the fused push and deposit, 256 x
+// 256 1.2, 128 x 128 2; with few particles (4 a cell) level.
+bool deposit_bands_fit(const Geom& g) {
+  constexpr int per = DT_MAX_SMEM / 8;
+  return g.ny <= per / 8 && (long long)g.nx * g.ny <= 8ll * per;
+}
+
+void launch_deposit_mixed_bands(cudaStream_t st, const Geom& g, const MixedSoA& p, const long long* d_n,
+                                unsigned long long* acc) {
+  const int most = DT_MAX_SMEM / 8 / g.ny - 1;  // cell rows that fit
+  const int want = (g.nx - 1 + most - 1) / most, rows = (g.nx - 1 + want - 1) / want;
+  const int bands = (g.nx - 1 + rows - 1) / rows;  // none is empty
+  int dev = 0, sms = 0;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  const int smem = (rows + 1) * g.ny * 8;
+  cudaFuncSetAttribute(k_deposit_mixed_bands, cudaFuncAttributeMaxDynamicSharedMemorySize, DT_MAX_SMEM);
+  k_deposit_mixed_bands<<<bands * std::max(1, sms / bands), DT_THREADS, smem, st>>>(g, p, d_n, acc, bands, rows);
+}
+
 // -------------------------------------------------------------- push ---
 // gather32 / advance / push_mixed_one: epic_mixed.cuh (shared with the batch).
 template <int SHAPE, int BC>
@@ -151,21 +262,22 @@ __global__ void __launch_bounds__(PART_THREADS) k_push_mixed(Geom g, MixedSoA p,
 // pass over the pushed electrons (mcc_candidate on the new velocities,
 // CTA-aggregated appends to sel.cand) in one pass over the particles.  Each
 // thread takes DEP_PER_THREAD consecutive particles with vector loads and
-// stores.  The particles, the integer sums and the candidate set (in another
+// stores.  Without DEP the deposit is left out (k_deposit_mixed_bands follows).
+// The particles, the integer sums and the candidate set (in another
 // order, which the MCC does not depend on) equal those of k_push_mixed +
 // k_deposit_mixed_sorted + k_mcc_select.
-template <int BC, bool SEL>
-__global__ void __launch_bounds__(PART_THREADS, 3) k_push_mixed_dep(Geom g, MixedSoA p, const long long* __restrict__ d_n,
+template <int BC, bool SEL, bool DEP>
+__global__ void __launch_bounds__(PART_THREADS, DEP ? 3 : 4) k_push_mixed_dep(Geom g, MixedSoA p, const long long* __restrict__ d_n,
                                                                  const float2* __restrict__ ef, float qmK_dt,
                                                                  float cx, float cy, unsigned long long* __restrict__ acc,
                                                                  SelectArgs sel) {
   constexpr int P = DEP_PER_THREAD;
-  __shared__ DepWarp tables[PART_THREADS / 32];
-  DepWarp& w = tables[threadIdx.x >> 5];
+  __shared__ DepWarp tables[DEP ? PART_THREADS / 32 : 1];
+  DepWarp& w = tables[DEP ? threadIdx.x >> 5 : 0];
   const long long n = *d_n;
   const unsigned long long step = SEL ? *sel.d_step : 0ull;
   const int lane = threadIdx.x & 31;
-  dep_init(w);
+  if (DEP) dep_init(w);
   for (long long chunk = (long long)blockIdx.x * DEP_CHUNK; chunk < n; chunk += (long long)gridDim.x * DEP_CHUNK) {
     const long long q0 = chunk + (long long)threadIdx.x * P;
     const bool full = q0 + P <= n;
@@ -245,7 +357,7 @@ __global__ void __launch_bounds__(PART_THREADS, 3) k_push_mixed_dep(Geom g, Mixe
       for (int k = 0; k < P; k++)
         if (cand & (1u << k)) sel.cand[o++] = (unsigned int)(q0 + k);
     }
-    deposit_warp_sorted(acc, w, ConstNy{g.ny}, c, ox, oy);
+    if (DEP) deposit_warp_sorted(acc, w, ConstNy{g.ny}, c, ox, oy);
   }
 }
 
@@ -318,7 +430,7 @@ __global__ void __launch_bounds__(PART_THREADS) k_push_mixed_compact(Geom g, Mix
 void launch_push_mixed(cudaStream_t st, const Geom& g, int shape, int bc, const MixedSoA& p, long long* d_n,
                        const float2* ef, float qmK_dt, float cx, float cy, int* flags,
                        unsigned long long* tile_status, unsigned int* tile_ctr, int grid,
-                       unsigned long long* dep_acc, const SelectArgs* sel, const CondSet* cond) {
+                       unsigned long long* dep_acc, const SelectArgs* sel, const CondSet* cond, bool bands) {
   if (cond) {  // the compacting push with the conductor test, for any wall rule
 #define PC(SH, B) \
   k_push_mixed_compact<SH, B, true><<<grid, PART_THREADS, 0, st>>>(g, p, d_n, ef, qmK_dt, cx, cy, tile_status, tile_ctr, \
@@ -339,11 +451,18 @@ void launch_push_mixed(cudaStream_t st, const Geom& g, int shape, int bc, const 
   if (dep_acc && shape == EPIC_CIC && (bc == EPIC_PBC || bc == EPIC_REFLECTIVE)) {
     const SelectArgs a = sel ? *sel : SelectArgs{};
     // one wave of resident CTAs (the kernel strides over the chunks)
-#define PD(B, S)                                                                                       \
-  k_push_mixed_dep<B, S><<<resident_grid(k_push_mixed_dep<B, S>, PART_THREADS), PART_THREADS, 0, st>>>( \
-      g, p, d_n, ef, qmK_dt, cx, cy, dep_acc, a)
+#define PD(B, S)                                                                                                   \
+  do {                                                                                                             \
+    if (bands)                                                                                                     \
+      k_push_mixed_dep<B, S, false><<<resident_grid(k_push_mixed_dep<B, S, false>, PART_THREADS), PART_THREADS, 0, \
+                                      st>>>(g, p, d_n, ef, qmK_dt, cx, cy, dep_acc, a);                            \
+    else                                                                                                           \
+      k_push_mixed_dep<B, S, true><<<resident_grid(k_push_mixed_dep<B, S, true>, PART_THREADS), PART_THREADS, 0,   \
+                                     st>>>(g, p, d_n, ef, qmK_dt, cx, cy, dep_acc, a);                             \
+  } while (0)
     if (bc == EPIC_PBC) { if (sel) PD(EPIC_PBC, true); else PD(EPIC_PBC, false); }
     else { if (sel) PD(EPIC_REFLECTIVE, true); else PD(EPIC_REFLECTIVE, false); }
+    if (bands) launch_deposit_mixed_bands(st, g, p, d_n, dep_acc);
 #undef PD
     return;
   }
