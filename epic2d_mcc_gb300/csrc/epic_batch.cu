@@ -133,13 +133,13 @@ __device__ __forceinline__ Geom run_geom(const BRun& r) {
 __global__ void __launch_bounds__(PART_THREADS) k_batch_push(const BRun* __restrict__ runs,
                                                              const int* __restrict__ node_run, MixedSoA p,
                                                              const long long* __restrict__ d_n,
-                                                             const float2* __restrict__ ef32, int s) {
+                                                             const FieldCell* __restrict__ ef32, int s) {
   const long long n = *d_n;
   for (long long q = (long long)blockIdx.x * blockDim.x + threadIdx.x; q < n; q += (long long)gridDim.x * blockDim.x) {
     const int cg = p.cell[q];
     const BRun& r = runs[node_run[cg]];
     const Geom g = run_geom(r);
-    const float2* ef = ef32 + r.node_off;
+    const FieldCell* ef = ef32 + r.node_off;
     int c = (int)(cg - r.node_off);
     float ox = p.ox[q], oy = p.oy[q], vx = p.vx[q], vy = p.vy[q];
     if (r.bc == EPIC_PBC) push_mixed_one<EPIC_CIC, EPIC_PBC>(g, ef, r.qmK_dt[s], r.cx, r.cy, c, ox, oy, vx, vy);
@@ -155,7 +155,7 @@ __global__ void __launch_bounds__(PART_THREADS) k_batch_push(const BRun* __restr
 __global__ void __launch_bounds__(PART_THREADS) k_batch_rewind(const BRun* __restrict__ runs,
                                                                const int* __restrict__ node_run, MixedSoA p,
                                                                const long long* __restrict__ d_n,
-                                                               const float2* __restrict__ ef32, int s) {
+                                                               const FieldCell* __restrict__ ef32, int s) {
   const long long n = *d_n;
   for (long long q = (long long)blockIdx.x * blockDim.x + threadIdx.x; q < n; q += (long long)gridDim.x * blockDim.x) {
     const int cg = p.cell[q];
@@ -187,7 +187,7 @@ template <bool SEL, int T>
 __global__ void __launch_bounds__(T, 768 / T) k_batch_push_dep(const BRun* __restrict__ runs,
                                                                     const int* __restrict__ node_run, MixedSoA p,
                                                                     const long long* __restrict__ d_n,
-                                                                    const float2* __restrict__ ef32, int s,
+                                                                    const FieldCell* __restrict__ ef32, int s,
                                                                     unsigned long long* __restrict__ acc,
                                                                     const unsigned long long* __restrict__ d_step,
                                                                     McEvents ev) {
@@ -259,7 +259,7 @@ __global__ void __launch_bounds__(T, 768 / T) k_batch_push_dep(const BRun* __res
           }
           rid = ri;
         }
-        const float2* ef = ef32 + roff;
+        const FieldCell* ef = ef32 + roff;
         int cl = (int)(c[k] - roff);
         if (rbc == EPIC_PBC)
           push_mixed_one<EPIC_CIC, EPIC_PBC>(g, ef, rqm, rcx, rcy, cl, ox[k], oy[k], vx[k], vy[k]);
@@ -322,7 +322,7 @@ __global__ void __launch_bounds__(T, 768 / T) k_batch_push_dep(const BRun* __res
 // every run's particles stay contiguous and in order.
 __global__ void __launch_bounds__(PART_THREADS) k_batch_push_compact(const BRun* __restrict__ runs,
                                                                      const int* __restrict__ node_run, MixedSoA p,
-                                                                     long long* d_n, const float2* __restrict__ ef32,
+                                                                     long long* d_n, const FieldCell* __restrict__ ef32,
                                                                      int s, unsigned long long* status,
                                                                      unsigned int* tile_ctr, int* flags, long long spin,
                                                                      BatchConductors cd) {
@@ -350,7 +350,7 @@ __global__ void __launch_bounds__(PART_THREADS) k_batch_push_compact(const BRun*
         const int run = __ldg(&node_run[cg]);
         const BRun& r = runs[run];
         const Geom g = run_geom(r);
-        const float2* ef = ef32 + r.node_off;
+        const FieldCell* ef = ef32 + r.node_off;
         int cl = (int)(cg - r.node_off);
         if (r.bc == EPIC_OPEN)
           keep[k] = push_mixed_one<EPIC_CIC, EPIC_OPEN>(g, ef, r.qmK_dt[s], r.cx, r.cy, cl, ox[k], oy[k], vx[k], vy[k]);
@@ -649,7 +649,7 @@ struct epic_batch {
   BRun* d_runs = nullptr;
   int* d_node_run = nullptr;
   double *phi = nullptr, *rho = nullptr, *efx = nullptr, *efy = nullptr;
-  float2* ef32 = nullptr;
+  FieldCell* ef32 = nullptr;
   MixedSoA arena[BATCH_MAX_SPECIES];
   long long* d_n[BATCH_MAX_SPECIES];
   long long cap[BATCH_MAX_SPECIES];
@@ -838,7 +838,7 @@ struct epic_batch {
   }
 
   template <bool SEL>
-  void launch_push(const MixedSoA& a, const long long* dn, const float2* ef, int s, unsigned long long* out, int T,
+  void launch_push(const MixedSoA& a, const long long* dn, const FieldCell* ef, int s, unsigned long long* out, int T,
                    int blocks) {
     if (T == 128)
       k_batch_push_dep<SEL, 128><<<blocks, 128, 0, stream>>>(d_runs, d_node_run, a, dn, ef, s, out, d_step, ev);
@@ -1079,7 +1079,7 @@ epic_status tune_particle_passes(epic_batch* b) {
   std::memset(&sm, 0, sizeof(sm));
   long long* dns = nullptr;
   unsigned long long* sacc = nullptr;
-  float2* zef = nullptr;
+  FieldCell* zef = nullptr;
   BCK(cudaMallocAsync((void**)&sm.cell, ns * sizeof(int), b->stream));
   BCK(cudaMallocAsync((void**)&sm.ox, ns * sizeof(float), b->stream));
   BCK(cudaMallocAsync((void**)&sm.oy, ns * sizeof(float), b->stream));
@@ -1088,7 +1088,7 @@ epic_status tune_particle_passes(epic_batch* b) {
   BCK(cudaMallocAsync((void**)&sm.vz, ns * sizeof(float), b->stream));
   BCK(cudaMallocAsync((void**)&dns, sizeof(long long), b->stream));
   BCK(cudaMallocAsync((void**)&sacc, b->nodes * sizeof(unsigned long long), b->stream));
-  BCK(cudaMallocAsync((void**)&zef, b->nodes * sizeof(float2), b->stream));
+  BCK(cudaMallocAsync((void**)&zef, b->nodes * sizeof(FieldCell), b->stream));
   const MixedSoA& a = b->arena[0];
   BCK(cudaMemcpyAsync(sm.cell, a.cell, ns * sizeof(int), cudaMemcpyDeviceToDevice, b->stream));
   BCK(cudaMemcpyAsync(sm.ox, a.ox, ns * sizeof(float), cudaMemcpyDeviceToDevice, b->stream));
@@ -1097,7 +1097,7 @@ epic_status tune_particle_passes(epic_batch* b) {
   BCK(cudaMemcpyAsync(sm.vy, a.vy, ns * sizeof(float), cudaMemcpyDeviceToDevice, b->stream));
   BCK(cudaMemcpyAsync(sm.vz, a.vz, ns * sizeof(float), cudaMemcpyDeviceToDevice, b->stream));
   BCK(cudaMemcpyAsync(dns, &ns, sizeof(long long), cudaMemcpyHostToDevice, b->stream));
-  BCK(cudaMemsetAsync(zef, 0, b->nodes * sizeof(float2), b->stream));
+  BCK(cudaMemsetAsync(zef, 0, b->nodes * sizeof(FieldCell), b->stream));
   cudaEvent_t e0, e1;
   cudaEventCreate(&e0);
   cudaEventCreate(&e1);

@@ -67,7 +67,7 @@ struct BatchGrids {
   const BRun* runs;
   const int* node_run;  // run of every node
   double *phi, *rho, *efx, *efy;
-  float2* ef32;
+  FieldCell* ef32;
   const unsigned long long* acc[BATCH_MAX_SPECIES];
 };
 

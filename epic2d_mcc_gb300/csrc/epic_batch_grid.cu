@@ -47,7 +47,7 @@ __global__ void k_batch_efield(BatchGrids b) {
     efield_node(xr, yr, nx, ny, r.dx, r.dy, PHI, i, j, ex, ey);
     b.efx[k] = ex;
     b.efy[k] = ey;
-    b.ef32[k] = make_float2((float)ex, (float)ey);
+    store_field_cell(b.ef32 + k, ny, i, j, make_float2((float)ex, (float)ey));
   }
 }
 

@@ -919,8 +919,11 @@ epic_status epic_create(const epic_config* cfg, epic_sim** out) {
   guard(dalloc(s, &s->rho, nn));
   guard(dalloc(s, &s->efx, nn));
   guard(dalloc(s, &s->efy, nn));
-  guard(dalloc(s, &s->ef, nn));
-  for (int k = 0; k < 8; k++) guard(dalloc(s, &s->work[k], nn));
+  s->mixed = cfg->precision == EPIC_PRECISION_MIXED;
+  if (!s->mixed) guard(dalloc(s, &s->ef, nn));
+  // the spectral solve has its own vectors; the last one's room goes to the field's records
+  const bool spectral = s->mixed && spectral_supported(s->g, cfg->solver, cfg->poisson_bc);
+  for (int k = 0; k < (spectral ? 7 : 8); k++) guard(dalloc(s, &s->work[k], nn));
   // Solver partials: up to 2 parities x 48 bytes per CTA (PCG), 16 doubles per CTA.
   guard(dalloc(s, &s->partials, 16 * (size_t)std::max(solver_max_blocks(), 320)));
   guard(dalloc(s, &s->bar, 2));
@@ -933,10 +936,9 @@ epic_status epic_create(const epic_config* cfg, epic_sim** out) {
   guard(dalloc(s, &s->d_sums, 4));
   guard(dalloc(s, &s->d_flags, 1));
   guard(dalloc(s, &s->d_nold, 2));
-  s->mixed = cfg->precision == EPIC_PRECISION_MIXED;
   if (s->mixed) {
     guard(dalloc(s, &s->ef32, nn));
-    if (spectral_supported(s->g, cfg->solver, cfg->poisson_bc) && !st) guard(setup_spectral(s));
+    if (spectral && !st) guard(setup_spectral(s));
   } else if (cfg->shape == EPIC_CIC && cfg->push_order == EPIC_PUSH_CONTRACTED) {
     guard(dalloc(s, &s->ef_cell, 4 * (size_t)nn));
   }
@@ -1833,14 +1835,19 @@ epic_status epic_set_grid(epic_sim* s, int which, const double* in) {
     CK(cudaStreamSynchronize(s->stream));
     std::vector<double2> e2(nnodes(s));
     for (long long k = 0; k < nnodes(s); k++) e2[k] = make_double2(ex[k], ey[k]);
-    CK(cudaMemcpyAsync(s->ef, e2.data(), nnodes(s) * sizeof(double2), cudaMemcpyHostToDevice, s->stream));
+    if (s->ef) CK(cudaMemcpyAsync(s->ef, e2.data(), nnodes(s) * sizeof(double2), cudaMemcpyHostToDevice, s->stream));
     if (s->ef_cell) launch_cell_coef(s->stream, s->g, s->ef, s->ef_cell);
     if (s->ef32) {
-      std::vector<float2> f2(nnodes(s));
-      for (long long k = 0; k < nnodes(s); k++) f2[k] = make_float2((float)ex[k], (float)ey[k]);
-      CK(cudaMemcpyAsync(s->ef32, f2.data(), nnodes(s) * sizeof(float2), cudaMemcpyHostToDevice, s->stream));
+      std::vector<FieldCell> f2(nnodes(s));
+      const long long ny = s->g.ny;
+      auto node = [&](long long k) {
+        return k < nnodes(s) ? make_float2((float)ex[k], (float)ey[k]) : make_float2(0.f, 0.f);
+      };
+      for (long long k = 0; k < nnodes(s); k++) f2[k] = {node(k), node(k + 1), node(k + ny), node(k + ny + 1)};
+      CK(cudaMemcpyAsync(s->ef32, f2.data(), nnodes(s) * sizeof(FieldCell), cudaMemcpyHostToDevice, s->stream));
+      CK(cudaStreamSynchronize(s->stream));  // f2 is a host temporary
     }
-    CK(cudaStreamSynchronize(s->stream));  // e2, f2 are host temporaries
+    CK(cudaStreamSynchronize(s->stream));  // e2 too
   }
   return EPIC_OK;
 }

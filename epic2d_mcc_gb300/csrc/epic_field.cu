@@ -79,7 +79,7 @@ void launch_finalize(cudaStream_t st, const FinalizeArgs& a) {
 // FieldSolve::CalculateEfield (src/field.cpp:276-330), edge rules xr, yr
 // (efield_edges).
 __global__ void k_efield(Geom g, int xr, int yr, const double* __restrict__ phi, double* efx, double* efy,
-                         double2* ef, float2* ef32) {
+                         double2* ef, FieldCell* ef32) {
   const int nx = g.nx, ny = g.ny;
   const int nn = nx * ny;
   for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < nn; k += gridDim.x * blockDim.x) {
@@ -89,13 +89,13 @@ __global__ void k_efield(Geom g, int xr, int yr, const double* __restrict__ phi,
     efield_node(xr, yr, nx, ny, g.dx, g.dy, PHI, i, j, ex, ey);
     efx[k] = ex;
     efy[k] = ey;
-    ef[k] = make_double2(ex, ey);
-    if (ef32) ef32[k] = make_float2((float)ex, (float)ey);
+    if (ef) ef[k] = make_double2(ex, ey);
+    if (ef32) store_field_cell(ef32 + k, ny, i, j, make_float2((float)ex, (float)ey));
   }
 }
 
 void launch_efield(cudaStream_t st, const Geom& g, int bc, int poisson_bc, const double* phi, double* efx,
-                   double* efy, double2* ef, float2* ef32) {
+                   double* efy, double2* ef, FieldCell* ef32) {
   int nn = g.nx * g.ny;
   int xr, yr;
   efield_edges(bc, poisson_bc, &xr, &yr);

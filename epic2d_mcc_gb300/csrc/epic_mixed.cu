@@ -242,7 +242,7 @@ void launch_deposit_mixed_bands(cudaStream_t st, const Geom& g, const MixedSoA& 
 // gather32 / advance / push_mixed_one: epic_mixed.cuh (shared with the batch).
 template <int SHAPE, int BC>
 __global__ void __launch_bounds__(PART_THREADS) k_push_mixed(Geom g, MixedSoA p, const long long* __restrict__ d_n,
-                                                             const float2* __restrict__ ef, float qmK_dt, float cx,
+                                                             const FieldCell* __restrict__ ef, float qmK_dt, float cx,
                                                              float cy) {
   const long long n = *d_n;
   for (long long q = (long long)blockIdx.x * blockDim.x + threadIdx.x; q < n; q += (long long)gridDim.x * blockDim.x) {
@@ -268,7 +268,7 @@ __global__ void __launch_bounds__(PART_THREADS) k_push_mixed(Geom g, MixedSoA p,
 // k_deposit_mixed_sorted + k_mcc_select.
 template <int BC, bool SEL, bool DEP>
 __global__ void __launch_bounds__(PART_THREADS, DEP ? 3 : 4) k_push_mixed_dep(Geom g, MixedSoA p, const long long* __restrict__ d_n,
-                                                                 const float2* __restrict__ ef, float qmK_dt,
+                                                                 const FieldCell* __restrict__ ef, float qmK_dt,
                                                                  float cx, float cy, unsigned long long* __restrict__ acc,
                                                                  SelectArgs sel) {
   constexpr int P = DEP_PER_THREAD;
@@ -368,7 +368,7 @@ __global__ void __launch_bounds__(PART_THREADS, DEP ? 3 : 4) k_push_mixed_dep(Ge
 // (src/species.cpp:80-165).
 template <int SHAPE, int BC, bool COND>
 __global__ void __launch_bounds__(PART_THREADS) k_push_mixed_compact(Geom g, MixedSoA p, long long* d_n,
-                                                                     const float2* __restrict__ ef, float qmK_dt,
+                                                                     const FieldCell* __restrict__ ef, float qmK_dt,
                                                                      float cx, float cy, unsigned long long* status,
                                                                      unsigned int* tile_ctr, int* flags,
                                                                      long long spin, CondSet cs) {
@@ -428,7 +428,7 @@ __global__ void __launch_bounds__(PART_THREADS) k_push_mixed_compact(Geom g, Mix
 }
 
 void launch_push_mixed(cudaStream_t st, const Geom& g, int shape, int bc, const MixedSoA& p, long long* d_n,
-                       const float2* ef, float qmK_dt, float cx, float cy, int* flags,
+                       const FieldCell* ef, float qmK_dt, float cx, float cy, int* flags,
                        unsigned long long* tile_status, unsigned int* tile_ctr, int grid,
                        unsigned long long* dep_acc, const SelectArgs* sel, const CondSet* cond, bool bands) {
   if (cond) {  // the compacting push with the conductor test, for any wall rule
@@ -486,7 +486,7 @@ void launch_push_mixed(cudaStream_t st, const Geom& g, int shape, int bc, const 
 // Species::Rewind_species (src/species.cpp:229-246): v -= (0.5*qm*K*DT) E.
 template <int SHAPE>
 __global__ void __launch_bounds__(PART_THREADS) k_rewind_mixed(Geom g, MixedSoA p, const long long* __restrict__ d_n,
-                                                               const float2* __restrict__ ef, float hqmK_dt) {
+                                                               const FieldCell* __restrict__ ef, float hqmK_dt) {
   const long long n = *d_n;
   for (long long q = (long long)blockIdx.x * blockDim.x + threadIdx.x; q < n; q += (long long)gridDim.x * blockDim.x) {
     float ex, ey;
@@ -497,7 +497,7 @@ __global__ void __launch_bounds__(PART_THREADS) k_rewind_mixed(Geom g, MixedSoA 
 }
 
 void launch_rewind_mixed(cudaStream_t st, const Geom& g, int shape, const MixedSoA& p, const long long* d_n,
-                         const float2* ef, float hqmK_dt, int* flags, int grid) {
+                         const FieldCell* ef, float hqmK_dt, int* flags, int grid) {
   (void)flags;
   if (shape == EPIC_NGP) k_rewind_mixed<EPIC_NGP><<<grid, PART_THREADS, 0, st>>>(g, p, d_n, ef, hqmK_dt);
   else k_rewind_mixed<EPIC_CIC><<<grid, PART_THREADS, 0, st>>>(g, p, d_n, ef, hqmK_dt);

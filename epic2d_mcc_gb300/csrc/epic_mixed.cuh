@@ -17,17 +17,19 @@ namespace epic {
 // boundary rule applied to the cell.  Periodic wrap is a modulo, so a
 // particle may cross any number of cells in a step.
 template <int SHAPE>
-__device__ __forceinline__ void gather32(const Geom& g, const float2* __restrict__ ef, int c, float ox, float oy,
+__device__ __forceinline__ void gather32(const Geom& g, const FieldCell* __restrict__ ef, int c, float ox, float oy,
                                          float& ex, float& ey) {
   if (SHAPE == EPIC_NGP) {
     const int k = c + (ox >= 0.5f ? g.ny : 0) + (oy >= 0.5f ? 1 : 0);
-    const float2 f = __ldg(&ef[k]);
+    const float2 f = __ldg(&ef[k].f00);
     ex = f.x;
     ey = f.y;
     return;
   }
-  const float2 f00 = __ldg(&ef[c]), f01 = __ldg(&ef[c + 1]);
-  const float2 f10 = __ldg(&ef[c + g.ny]), f11 = __ldg(&ef[c + g.ny + 1]);
+  float2 f00, f01, f10, f11;
+  asm("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+      : "=f"(f00.x), "=f"(f00.y), "=f"(f01.x), "=f"(f01.y), "=f"(f10.x), "=f"(f10.y), "=f"(f11.x), "=f"(f11.y)
+      : "l"(ef + c));
   const float w00 = (1.f - ox) * (1.f - oy), w10 = ox * (1.f - oy), w01 = (1.f - ox) * oy, w11 = ox * oy;
   ex = f00.x * w00 + f10.x * w10 + f01.x * w01 + f11.x * w11;
   ey = f00.y * w00 + f10.y * w10 + f01.y * w01 + f11.y * w11;
@@ -117,7 +119,7 @@ __device__ __forceinline__ bool advance(int& idx, float& o, float& v, float d, i
 }
 
 template <int SHAPE, int BC>
-__device__ __forceinline__ bool push_mixed_one(const Geom& g, const float2* __restrict__ ef, float qmK_dt, float cx,
+__device__ __forceinline__ bool push_mixed_one(const Geom& g, const FieldCell* __restrict__ ef, float qmK_dt, float cx,
                                                float cy, int& c, float& ox, float& oy, float& vx, float& vy) {
   float ex, ey;
   gather32<SHAPE>(g, ef, c, ox, oy, ex, ey);
