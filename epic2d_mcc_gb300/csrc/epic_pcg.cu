@@ -182,7 +182,7 @@ constexpr unsigned long long PM_OUT = (1ull << 62) - 1;
 // 64 x 64-bit high product takes ~40 cycles of the integer pipe, an FP64 product
 // holds the warp's quarter of the SM for 64 and its result would have to be
 // taken apart again (an iteration at 257 x 257: 1.89 us with FP64 products,
-// 1.82 us so; with 16 components a thread, 1024 x 1024: 7.0 against 6.0 us).
+// 1.82 us so; with 16 components a thread, 1024 x 1024: 6.8 against 6.0 us).
 // Cut at 2^-62 of the term, where an FP64 product is rounded at 2^-53.
 __device__ __forceinline__ void pm_terms(unsigned long long& v0, unsigned long long& v1, bool& b0, bool& b1, double r,
                                          double L, int E0, int E1) {
