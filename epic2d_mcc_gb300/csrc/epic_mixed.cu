@@ -280,39 +280,39 @@ __global__ void __launch_bounds__(PART_THREADS, DEP ? 3 : 4) k_push_mixed_dep(Ge
   const int lane = threadIdx.x & 31;
   if (DEP) dep_init(w);
   for (long long chunk = (long long)blockIdx.x * DEP_CHUNK; chunk < n; chunk += (long long)gridDim.x * DEP_CHUNK) {
-    const long long q0 = chunk + (long long)threadIdx.x * P;
-    const bool full = q0 + P <= n;
+    const long long q0 = chunk + (threadIdx.x >> 5) * DEP_WARP_CHUNK + 4 * lane;  // and 128 further, ...
     int c[P];
     float ox[P], oy[P], vx[P], vy[P], vz[P];
-    if (full) {
 #pragma unroll
-      for (int h = 0; h < P / 4; h++) {
-        const int4 cc = reinterpret_cast<const int4*>(p.cell + q0)[h];
-        const float4 a = reinterpret_cast<const float4*>(p.ox + q0)[h];
-        const float4 b = reinterpret_cast<const float4*>(p.oy + q0)[h];
-        const float4 u = reinterpret_cast<const float4*>(p.vx + q0)[h];
-        const float4 v = reinterpret_cast<const float4*>(p.vy + q0)[h];
-        c[4 * h] = cc.x; c[4 * h + 1] = cc.y; c[4 * h + 2] = cc.z; c[4 * h + 3] = cc.w;
-        ox[4 * h] = a.x; ox[4 * h + 1] = a.y; ox[4 * h + 2] = a.z; ox[4 * h + 3] = a.w;
-        oy[4 * h] = b.x; oy[4 * h + 1] = b.y; oy[4 * h + 2] = b.z; oy[4 * h + 3] = b.w;
-        vx[4 * h] = u.x; vx[4 * h + 1] = u.y; vx[4 * h + 2] = u.z; vx[4 * h + 3] = u.w;
-        vy[4 * h] = v.x; vy[4 * h + 1] = v.y; vy[4 * h + 2] = v.z; vy[4 * h + 3] = v.w;
+    for (int h = 0; h < P; h += 4) {
+      const long long q = q0 + 32 * h;
+      if (q + 4 <= n) {
+        const int4 cc = *reinterpret_cast<const int4*>(p.cell + q);
+        const float4 a = *reinterpret_cast<const float4*>(p.ox + q);
+        const float4 b = *reinterpret_cast<const float4*>(p.oy + q);
+        const float4 u = *reinterpret_cast<const float4*>(p.vx + q);
+        const float4 v = *reinterpret_cast<const float4*>(p.vy + q);
+        c[h] = cc.x; c[h + 1] = cc.y; c[h + 2] = cc.z; c[h + 3] = cc.w;
+        ox[h] = a.x; ox[h + 1] = a.y; ox[h + 2] = a.z; ox[h + 3] = a.w;
+        oy[h] = b.x; oy[h + 1] = b.y; oy[h + 2] = b.z; oy[h + 3] = b.w;
+        vx[h] = u.x; vx[h + 1] = u.y; vx[h + 2] = u.z; vx[h + 3] = u.w;
+        vy[h] = v.x; vy[h + 1] = v.y; vy[h + 2] = v.z; vy[h + 3] = v.w;
         if (SEL) {
-          const float4 w = reinterpret_cast<const float4*>(p.vz + q0)[h];
-          vz[4 * h] = w.x; vz[4 * h + 1] = w.y; vz[4 * h + 2] = w.z; vz[4 * h + 3] = w.w;
+          const float4 w = *reinterpret_cast<const float4*>(p.vz + q);
+          vz[h] = w.x; vz[h + 1] = w.y; vz[h + 2] = w.z; vz[h + 3] = w.w;
         }
-      }
-    } else {
+      } else {
 #pragma unroll
-      for (int k = 0; k < P; k++) {
-        const long long q = q0 + k;
-        const bool in = q < n;
-        c[k] = in ? p.cell[q] : -1;
-        ox[k] = in ? p.ox[q] : 0.f;
-        oy[k] = in ? p.oy[q] : 0.f;
-        vx[k] = in ? p.vx[q] : 0.f;
-        vy[k] = in ? p.vy[q] : 0.f;
-        vz[k] = (SEL && in) ? p.vz[q] : 0.f;
+        for (int k = h; k < h + 4; k++) {
+          const long long m = q + k - h;
+          const bool in = m < n;
+          c[k] = in ? p.cell[m] : -1;
+          ox[k] = in ? p.ox[m] : 0.f;
+          oy[k] = in ? p.oy[m] : 0.f;
+          vx[k] = in ? p.vx[m] : 0.f;
+          vy[k] = in ? p.vy[m] : 0.f;
+          vz[k] = (SEL && in) ? p.vz[m] : 0.f;
+        }
       }
     }
     unsigned int cand = 0;
@@ -320,28 +320,29 @@ __global__ void __launch_bounds__(PART_THREADS, DEP ? 3 : 4) k_push_mixed_dep(Ge
     for (int k = 0; k < P; k++)
       if (c[k] >= 0) {
         push_mixed_one<EPIC_CIC, BC>(g, ef, qmK_dt, cx, cy, c[k], ox[k], oy[k], vx[k], vy[k]);
-        if (SEL && mcc_candidate(sel, q0 + k, step, vx[k], vy[k], vz[k])) cand |= 1u << k;
+        if (SEL && mcc_candidate(sel, q0 + 31 * (k & ~3) + k, step, vx[k], vy[k], vz[k])) cand |= 1u << k;
       }
-    if (full) {
 #pragma unroll
-      for (int h = 0; h < P / 4; h++) {
-        reinterpret_cast<int4*>(p.cell + q0)[h] = make_int4(c[4 * h], c[4 * h + 1], c[4 * h + 2], c[4 * h + 3]);
-        reinterpret_cast<float4*>(p.ox + q0)[h] = make_float4(ox[4 * h], ox[4 * h + 1], ox[4 * h + 2], ox[4 * h + 3]);
-        reinterpret_cast<float4*>(p.oy + q0)[h] = make_float4(oy[4 * h], oy[4 * h + 1], oy[4 * h + 2], oy[4 * h + 3]);
-        reinterpret_cast<float4*>(p.vx + q0)[h] = make_float4(vx[4 * h], vx[4 * h + 1], vx[4 * h + 2], vx[4 * h + 3]);
-        reinterpret_cast<float4*>(p.vy + q0)[h] = make_float4(vy[4 * h], vy[4 * h + 1], vy[4 * h + 2], vy[4 * h + 3]);
+    for (int h = 0; h < P; h += 4) {
+      const long long q = q0 + 32 * h;
+      if (q + 4 <= n) {
+        *reinterpret_cast<int4*>(p.cell + q) = make_int4(c[h], c[h + 1], c[h + 2], c[h + 3]);
+        *reinterpret_cast<float4*>(p.ox + q) = make_float4(ox[h], ox[h + 1], ox[h + 2], ox[h + 3]);
+        *reinterpret_cast<float4*>(p.oy + q) = make_float4(oy[h], oy[h + 1], oy[h + 2], oy[h + 3]);
+        *reinterpret_cast<float4*>(p.vx + q) = make_float4(vx[h], vx[h + 1], vx[h + 2], vx[h + 3]);
+        *reinterpret_cast<float4*>(p.vy + q) = make_float4(vy[h], vy[h + 1], vy[h + 2], vy[h + 3]);
+      } else {
+#pragma unroll
+        for (int k = h; k < h + 4; k++)
+          if (c[k] >= 0) {
+            const long long m = q + k - h;
+            p.cell[m] = c[k];
+            p.ox[m] = ox[k];
+            p.oy[m] = oy[k];
+            p.vx[m] = vx[k];
+            p.vy[m] = vy[k];
+          }
       }
-    } else {
-#pragma unroll
-      for (int k = 0; k < P; k++)
-        if (c[k] >= 0) {
-          const long long q = q0 + k;
-          p.cell[q] = c[k];
-          p.ox[q] = ox[k];
-          p.oy[q] = oy[k];
-          p.vx[q] = vx[k];
-          p.vy[q] = vy[k];
-        }
     }
     if (SEL && __any_sync(0xffffffffu, cand != 0)) {  // one atomic per warp with candidates
       const unsigned int mine = __popc(cand);
@@ -356,7 +357,7 @@ __global__ void __launch_bounds__(PART_THREADS, DEP ? 3 : 4) k_push_mixed_dep(Ge
       unsigned int o = __shfl_sync(0xffffffffu, base, 31) + incl - mine;
 #pragma unroll
       for (int k = 0; k < P; k++)
-        if (cand & (1u << k)) sel.cand[o++] = (unsigned int)(q0 + k);
+        if (cand & (1u << k)) sel.cand[o++] = (unsigned int)(q0 + 31 * (k & ~3) + k);
     }
     if (DEP) deposit_warp_sorted(acc, w, ConstNy{g.ny}, c, ox, oy);
   }
