@@ -175,10 +175,15 @@ __global__ void __launch_bounds__(PART_THREADS) k_batch_rewind(const BRun* __res
 // runs (appended to ev.cand, one atomic per warp with candidates).  Particles,
 // integer sums and the candidate set equal k_batch_push + k_batch_deposit +
 // k_batch_mcc_select.
+// The row stride of the run that holds a cell: that of the lane's current run
+// (nodes [lo, lo + span)) without a look at the tables.
 struct RunNy {
   const BRun* runs;
   const int* node_run;
-  __device__ __forceinline__ int operator()(int cg) const { return runs[__ldg(&node_run[cg])].ny; }
+  int lo = 0, span = 0, ny = 0;
+  __device__ __forceinline__ int operator()(int cg) const {
+    return (unsigned)(cg - lo) < (unsigned)span ? ny : runs[__ldg(&node_run[cg])].ny;
+  }
 };
 
 // T threads per CTA (128 or 256; the autotuner picks the shape), each taking
@@ -198,56 +203,57 @@ __global__ void __launch_bounds__(T, 768 / T) k_batch_push_dep(const BRun* __res
   const long long n = *d_n;
   const unsigned long long step = SEL ? *d_step : 0ull;
   const int lane = threadIdx.x & 31;
-  const RunNy ny_of{runs, node_run};
+  RunNy at{runs, node_run};
   dep_init(w);
+  // A lane's particles are near each other in the cell-sorted array, so they
+  // nearly always share a run, from chunk to chunk too: its parameters are
+  // loaded once and kept while the run stays the same.
+  int rnx = 0, rbc = 0, rmcc = 0;
+  unsigned rinv = 0;
+  float rqm = 0.f, rcx = 0.f, rcy = 0.f;
+  unsigned long long rcut = 0, rseed = 0;
   for (long long chunk = (long long)blockIdx.x * CHUNK; chunk < n; chunk += (long long)gridDim.x * CHUNK) {
-    const long long q0 = chunk + (long long)threadIdx.x * P;
-    const bool full = q0 + P <= n;
+    const long long q0 = chunk + (threadIdx.x >> 5) * DEP_WARP_CHUNK + 4 * lane;  // and 128 further, ...
     int c[P];
     float ox[P], oy[P], vx[P], vy[P];
-    if (full) {
 #pragma unroll
-      for (int h = 0; h < P / 4; h++) {
-        const int4 cc = reinterpret_cast<const int4*>(p.cell + q0)[h];
-        const float4 a = reinterpret_cast<const float4*>(p.ox + q0)[h];
-        const float4 b = reinterpret_cast<const float4*>(p.oy + q0)[h];
-        const float4 u = reinterpret_cast<const float4*>(p.vx + q0)[h];
-        const float4 v = reinterpret_cast<const float4*>(p.vy + q0)[h];
-        c[4 * h] = cc.x; c[4 * h + 1] = cc.y; c[4 * h + 2] = cc.z; c[4 * h + 3] = cc.w;
-        ox[4 * h] = a.x; ox[4 * h + 1] = a.y; ox[4 * h + 2] = a.z; ox[4 * h + 3] = a.w;
-        oy[4 * h] = b.x; oy[4 * h + 1] = b.y; oy[4 * h + 2] = b.z; oy[4 * h + 3] = b.w;
-        vx[4 * h] = u.x; vx[4 * h + 1] = u.y; vx[4 * h + 2] = u.z; vx[4 * h + 3] = u.w;
-        vy[4 * h] = v.x; vy[4 * h + 1] = v.y; vy[4 * h + 2] = v.z; vy[4 * h + 3] = v.w;
-      }
-    } else {
+    for (int h = 0; h < P; h += 4) {
+      const long long q = q0 + 32 * h;
+      if (q + 4 <= n) {
+        const int4 cc = *reinterpret_cast<const int4*>(p.cell + q);
+        const float4 a = *reinterpret_cast<const float4*>(p.ox + q);
+        const float4 b = *reinterpret_cast<const float4*>(p.oy + q);
+        const float4 u = *reinterpret_cast<const float4*>(p.vx + q);
+        const float4 v = *reinterpret_cast<const float4*>(p.vy + q);
+        c[h] = cc.x; c[h + 1] = cc.y; c[h + 2] = cc.z; c[h + 3] = cc.w;
+        ox[h] = a.x; ox[h + 1] = a.y; ox[h + 2] = a.z; ox[h + 3] = a.w;
+        oy[h] = b.x; oy[h + 1] = b.y; oy[h + 2] = b.z; oy[h + 3] = b.w;
+        vx[h] = u.x; vx[h + 1] = u.y; vx[h + 2] = u.z; vx[h + 3] = u.w;
+        vy[h] = v.x; vy[h + 1] = v.y; vy[h + 2] = v.z; vy[h + 3] = v.w;
+      } else {
 #pragma unroll
-      for (int k = 0; k < P; k++) {
-        const long long q = q0 + k;
-        const bool in = q < n;
-        c[k] = in ? p.cell[q] : -1;
-        ox[k] = in ? p.ox[q] : 0.f;
-        oy[k] = in ? p.oy[q] : 0.f;
-        vx[k] = in ? p.vx[q] : 0.f;
-        vy[k] = in ? p.vy[q] : 0.f;
+        for (int k = h; k < h + 4; k++) {
+          const long long m = q + k - h;
+          const bool in = m < n;
+          c[k] = in ? p.cell[m] : -1;
+          ox[k] = in ? p.ox[m] : 0.f;
+          oy[k] = in ? p.oy[m] : 0.f;
+          vx[k] = in ? p.vx[m] : 0.f;
+          vy[k] = in ? p.vy[m] : 0.f;
+        }
       }
     }
     unsigned int cand = 0;
-    // A thread's particles are consecutive in the cell-sorted array, so they
-    // nearly always share a run: its parameters are loaded once and kept
-    // while the run stays the same.
-    int rid = -1, rbc = 0, rmcc = 0;
-    long long roff = 0;
-    float rqm = 0.f, rcx = 0.f, rcy = 0.f;
-    unsigned long long rcut = 0, rseed = 0;
-    Geom g;
 #pragma unroll
     for (int k = 0; k < P; k++)
       if (c[k] >= 0) {
-        const int ri = __ldg(&node_run[c[k]]);
-        if (ri != rid) {
-          const BRun& r = runs[ri];
-          g = run_geom(r);
-          roff = r.node_off;
+        if ((unsigned)(c[k] - at.lo) >= (unsigned)at.span) {
+          const BRun& r = runs[__ldg(&node_run[c[k]])];
+          at.lo = (int)r.node_off;
+          at.span = r.nx * r.ny;
+          at.ny = r.ny;
+          rnx = r.nx;
+          rinv = 0xFFFFFFFFu / (unsigned)r.ny;
           rbc = r.bc;
           rqm = r.qmK_dt[s];
           rcx = r.cx;
@@ -257,42 +263,43 @@ __global__ void __launch_bounds__(T, 768 / T) k_batch_push_dep(const BRun* __res
             rcut = r.cut53;
             rseed = r.seed;
           }
-          rid = ri;
         }
-        const FieldCell* ef = ef32 + roff;
-        int cl = (int)(c[k] - roff);
+        float ex, ey;
+        gather_cell32(load_cell32(ef32 + c[k]), ox[k], oy[k], ex, ey);
+        int cl = c[k] - at.lo;
         if (rbc == EPIC_PBC)
-          push_mixed_one<EPIC_CIC, EPIC_PBC>(g, ef, rqm, rcx, rcy, cl, ox[k], oy[k], vx[k], vy[k]);
+          push_mixed_in<EPIC_PBC>(rnx, at.ny, rinv, ex, ey, rqm, rcx, rcy, cl, ox[k], oy[k], vx[k], vy[k]);
         else
-          push_mixed_one<EPIC_CIC, EPIC_REFLECTIVE>(g, ef, rqm, rcx, rcy, cl, ox[k], oy[k], vx[k], vy[k]);
-        c[k] = (int)(roff + cl);
+          push_mixed_in<EPIC_REFLECTIVE>(rnx, at.ny, rinv, ex, ey, rqm, rcx, rcy, cl, ox[k], oy[k], vx[k], vy[k]);
+        c[k] = at.lo + cl;
         if (SEL && rmcc) {
-          const long long q = q0 + k;
+          const long long q = q0 + 31 * (k & ~3) + k;
           Philox src{(uint32_t)q, (uint32_t)(q >> 32), (uint32_t)step, (uint32_t)rseed, (uint32_t)(rseed >> 32), 0,
                      make_uint4(0, 0, 0, 0)};
           if (src.next53() < rcut) cand |= 1u << k;
         }
       }
-    if (full) {
 #pragma unroll
-      for (int h = 0; h < P / 4; h++) {
-        reinterpret_cast<int4*>(p.cell + q0)[h] = make_int4(c[4 * h], c[4 * h + 1], c[4 * h + 2], c[4 * h + 3]);
-        reinterpret_cast<float4*>(p.ox + q0)[h] = make_float4(ox[4 * h], ox[4 * h + 1], ox[4 * h + 2], ox[4 * h + 3]);
-        reinterpret_cast<float4*>(p.oy + q0)[h] = make_float4(oy[4 * h], oy[4 * h + 1], oy[4 * h + 2], oy[4 * h + 3]);
-        reinterpret_cast<float4*>(p.vx + q0)[h] = make_float4(vx[4 * h], vx[4 * h + 1], vx[4 * h + 2], vx[4 * h + 3]);
-        reinterpret_cast<float4*>(p.vy + q0)[h] = make_float4(vy[4 * h], vy[4 * h + 1], vy[4 * h + 2], vy[4 * h + 3]);
+    for (int h = 0; h < P; h += 4) {
+      const long long q = q0 + 32 * h;
+      if (q + 4 <= n) {
+        *reinterpret_cast<int4*>(p.cell + q) = make_int4(c[h], c[h + 1], c[h + 2], c[h + 3]);
+        *reinterpret_cast<float4*>(p.ox + q) = make_float4(ox[h], ox[h + 1], ox[h + 2], ox[h + 3]);
+        *reinterpret_cast<float4*>(p.oy + q) = make_float4(oy[h], oy[h + 1], oy[h + 2], oy[h + 3]);
+        *reinterpret_cast<float4*>(p.vx + q) = make_float4(vx[h], vx[h + 1], vx[h + 2], vx[h + 3]);
+        *reinterpret_cast<float4*>(p.vy + q) = make_float4(vy[h], vy[h + 1], vy[h + 2], vy[h + 3]);
+      } else {
+#pragma unroll
+        for (int k = h; k < h + 4; k++)
+          if (c[k] >= 0) {
+            const long long m = q + k - h;
+            p.cell[m] = c[k];
+            p.ox[m] = ox[k];
+            p.oy[m] = oy[k];
+            p.vx[m] = vx[k];
+            p.vy[m] = vy[k];
+          }
       }
-    } else {
-#pragma unroll
-      for (int k = 0; k < P; k++)
-        if (c[k] >= 0) {
-          const long long q = q0 + k;
-          p.cell[q] = c[k];
-          p.ox[q] = ox[k];
-          p.oy[q] = oy[k];
-          p.vx[q] = vx[k];
-          p.vy[q] = vy[k];
-        }
     }
     if (SEL && __any_sync(0xffffffffu, cand != 0)) {
       const unsigned int mine = __popc(cand);
@@ -307,9 +314,9 @@ __global__ void __launch_bounds__(T, 768 / T) k_batch_push_dep(const BRun* __res
       unsigned int o = __shfl_sync(0xffffffffu, base, 31) + incl - mine;
 #pragma unroll
       for (int k = 0; k < P; k++)
-        if (cand & (1u << k)) ev.cand[o++] = (unsigned int)(q0 + k);
+        if (cand & (1u << k)) ev.cand[o++] = (unsigned int)(q0 + 31 * (k & ~3) + k);
     }
-    deposit_warp_sorted(acc, w, ny_of, c, ox, oy);
+    deposit_warp_sorted(acc, w, at, c, ox, oy);
   }
 }
 

@@ -268,7 +268,7 @@ __global__ void __launch_bounds__(PART_THREADS) k_push_mixed(Geom g, MixedSoA p,
 // order, which the MCC does not depend on) equal those of k_push_mixed +
 // k_deposit_mixed_sorted + k_mcc_select.
 template <int BC, bool SEL, bool DEP>
-__global__ void __launch_bounds__(PART_THREADS, DEP ? 3 : 4) k_push_mixed_dep(Geom g, MixedSoA p, const long long* __restrict__ d_n,
+__global__ void __launch_bounds__(PART_THREADS, 3) k_push_mixed_dep(Geom g, MixedSoA p, const long long* __restrict__ d_n,
                                                                  const FieldCell* __restrict__ ef, float qmK_dt,
                                                                  float cx, float cy, unsigned long long* __restrict__ acc,
                                                                  SelectArgs sel) {

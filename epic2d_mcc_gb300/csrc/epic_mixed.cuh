@@ -16,6 +16,19 @@ namespace epic {
 // then whole cells are carried from the offset into the cell index and the
 // boundary rule applied to the cell.  Periodic wrap is a modulo, so a
 // particle may cross any number of cells in a step.
+__device__ __forceinline__ FieldCell load_cell32(const FieldCell* at) {
+  FieldCell f;
+  asm("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+      : "=f"(f.f00.x), "=f"(f.f00.y), "=f"(f.f01.x), "=f"(f.f01.y), "=f"(f.f10.x), "=f"(f.f10.y), "=f"(f.f11.x),
+        "=f"(f.f11.y)
+      : "l"(at));
+  return f;
+}
+__device__ __forceinline__ void gather_cell32(const FieldCell& f, float ox, float oy, float& ex, float& ey) {
+  const float w00 = (1.f - ox) * (1.f - oy), w10 = ox * (1.f - oy), w01 = (1.f - ox) * oy, w11 = ox * oy;
+  ex = f.f00.x * w00 + f.f10.x * w10 + f.f01.x * w01 + f.f11.x * w11;
+  ey = f.f00.y * w00 + f.f10.y * w10 + f.f01.y * w01 + f.f11.y * w11;
+}
 template <int SHAPE>
 __device__ __forceinline__ void gather32(const Geom& g, const FieldCell* __restrict__ ef, int c, float ox, float oy,
                                          float& ex, float& ey) {
@@ -26,13 +39,7 @@ __device__ __forceinline__ void gather32(const Geom& g, const FieldCell* __restr
     ey = f.y;
     return;
   }
-  float2 f00, f01, f10, f11;
-  asm("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
-      : "=f"(f00.x), "=f"(f00.y), "=f"(f01.x), "=f"(f01.y), "=f"(f10.x), "=f"(f10.y), "=f"(f11.x), "=f"(f11.y)
-      : "l"(ef + c));
-  const float w00 = (1.f - ox) * (1.f - oy), w10 = ox * (1.f - oy), w01 = (1.f - ox) * oy, w11 = ox * oy;
-  ex = f00.x * w00 + f10.x * w10 + f01.x * w01 + f11.x * w11;
-  ey = f00.y * w00 + f10.y * w10 + f01.y * w01 + f11.y * w11;
+  gather_cell32(load_cell32(ef + c), ox, oy, ex, ey);
 }
 
 // The largest FP32 offset below 1: a particle inside the domain whose offset
@@ -63,8 +70,7 @@ __device__ __forceinline__ bool cell_offset(double l, int ncell, int& idx, float
 // c = i * ny + j, 0 <= c < 2^31, 0 < ny: (i, j) with a multiply-high
 // (m = floor((2^32 - 1) / ny) underestimates 1/ny by less than 2^-32, so the
 // quotient is exact or one short) in place of an integer division.
-__device__ __forceinline__ void split_cell(int c, int ny, int& i, int& j) {
-  const unsigned m = 0xFFFFFFFFu / (unsigned)ny;  // loop-invariant
+__device__ __forceinline__ void split_cell(int c, int ny, unsigned m, int& i, int& j) {
   unsigned q = __umulhi((unsigned)c, m);
   int r = c - (int)q * ny;
   if (r >= ny) {
@@ -73,6 +79,9 @@ __device__ __forceinline__ void split_cell(int c, int ny, int& i, int& j) {
   }
   i = (int)q;
   j = r;
+}
+__device__ __forceinline__ void split_cell(int c, int ny, int& i, int& j) {
+  split_cell(c, ny, 0xFFFFFFFFu / (unsigned)ny, i, j);  // loop-invariant where ny is
 }
 
 // Moves (cell index, offset) along one axis by `d` cells and applies the
@@ -118,19 +127,26 @@ __device__ __forceinline__ bool advance(int& idx, float& o, float& v, float d, i
   }
 }
 
+// The push in the field (ex, ey) at the particle; inv: split_cell's m.
+template <int BC>
+__device__ __forceinline__ bool push_mixed_in(int nx, int ny, unsigned inv, float ex, float ey, float qmK_dt, float cx,
+                                              float cy, int& c, float& ox, float& oy, float& vx, float& vy) {
+  vx = fmaf(qmK_dt, ex, vx);
+  vy = fmaf(qmK_dt, ey, vy);
+  int i, j;
+  split_cell(c, ny, inv, i, j);
+  bool keep = advance<BC>(i, ox, vx, cx * vx, nx - 1);
+  keep = advance<BC>(j, oy, vy, cy * vy, ny - 1) && keep;
+  c = i * ny + j;
+  return keep;
+}
+
 template <int SHAPE, int BC>
 __device__ __forceinline__ bool push_mixed_one(const Geom& g, const FieldCell* __restrict__ ef, float qmK_dt, float cx,
                                                float cy, int& c, float& ox, float& oy, float& vx, float& vy) {
   float ex, ey;
   gather32<SHAPE>(g, ef, c, ox, oy, ex, ey);
-  vx = fmaf(qmK_dt, ex, vx);
-  vy = fmaf(qmK_dt, ey, vy);
-  int i, j;
-  split_cell(c, g.ny, i, j);
-  bool keep = advance<BC>(i, ox, vx, cx * vx, g.nx - 1);
-  keep = advance<BC>(j, oy, vy, cy * vy, g.ny - 1) && keep;
-  c = i * g.ny + j;
-  return keep;
+  return push_mixed_in<BC>(g.nx, g.ny, 0xFFFFFFFFu / (unsigned)g.ny, ex, ey, qmK_dt, cx, cy, c, ox, oy, vx, vy);
 }
 
 // ------------------------------------------ deposit of a sorted chunk ---
