@@ -53,12 +53,6 @@ __global__ void k_sort_keys_fp64(Geom g, SoA p, const long long* __restrict__ d_
   }
 }
 
-__global__ void k_sort_keys_mixed(MixedSoA p, const long long* __restrict__ d_n, unsigned* __restrict__ keys) {
-  const long long n = *d_n;
-  for (long long q = (long long)blockIdx.x * blockDim.x + threadIdx.x; q < n; q += (long long)gridDim.x * blockDim.x)
-    keys[q] = (unsigned)p.cell[q];
-}
-
 // Digit counts of one tile: hist[d * T + tile].
 __global__ void __launch_bounds__(SORT_T) k_radix_hist(const unsigned* __restrict__ keys,
                                                       const long long* __restrict__ d_n, int shift,
@@ -68,9 +62,28 @@ __global__ void __launch_bounds__(SORT_T) k_radix_hist(const unsigned* __restric
   __syncthreads();
   const long long n = *d_n;
   const long long base = (long long)blockIdx.x * SORT_TILE;
-  for (int m = threadIdx.x; m < SORT_TILE; m += SORT_T) {
+  // four consecutive keys a thread, equal neighbours counted together: between
+  // sorts the keys are nearly in order, and a warp's would all add to one digit
+  for (int m = 4 * threadIdx.x; m < SORT_TILE; m += 4 * SORT_T) {
     const long long q = base + m;
-    if (q < n) atomicAdd(&cnt[(keys[q] >> shift) & (RADIX - 1)], 1u);
+    if (q + 4 <= n) {
+      const uint4 k = *reinterpret_cast<const uint4*>(keys + q);
+      const unsigned d[4] = {(k.x >> shift) & (RADIX - 1), (k.y >> shift) & (RADIX - 1), (k.z >> shift) & (RADIX - 1),
+                             (k.w >> shift) & (RADIX - 1)};
+      unsigned run = 1;
+#pragma unroll
+      for (int i = 0; i < 4; i++) {
+        if (i < 3 && d[i] == d[(i + 1) & 3]) {
+          run++;
+        } else {
+          atomicAdd(&cnt[d[i]], run);
+          run = 1;
+        }
+      }
+    } else {
+      for (int i = 0; i < 4; i++)
+        if (q + i < n) atomicAdd(&cnt[(keys[q + i] >> shift) & (RADIX - 1)], 1u);
+    }
   }
   __syncthreads();
   for (int d = threadIdx.x; d < RADIX; d += SORT_T) hist[(long long)d * T + blockIdx.x] = cnt[d];
@@ -234,29 +247,70 @@ __global__ void k_copy_fp64(SoA tmp, SoA dst, const long long* __restrict__ d_n)
   }
 }
 
-__global__ void k_gather_mixed(MixedSoA src, MixedSoA tmp, const unsigned* __restrict__ perm,
-                               const long long* __restrict__ d_n) {
+// Four particles a thread: 20 gathers in flight, 16-byte stores.  The cells are
+// the sorted keys themselves.  5.2e7 nearly sorted particles: 1.05 ms one at a
+// time, 0.35 so; the copy back 0.59 and 0.38.
+__global__ void __launch_bounds__(PART_THREADS) k_gather_mixed(MixedSoA src, MixedSoA tmp,
+                                                               const unsigned* __restrict__ perm,
+                                                               const long long* __restrict__ d_n) {
   const long long n = *d_n;
-  for (long long q = (long long)blockIdx.x * blockDim.x + threadIdx.x; q < n; q += (long long)gridDim.x * blockDim.x) {
-    const unsigned j = perm[q];
-    tmp.cell[q] = src.cell[j];
-    tmp.ox[q] = src.ox[j];
-    tmp.oy[q] = src.oy[j];
-    tmp.vx[q] = src.vx[j];
-    tmp.vy[q] = src.vy[j];
-    tmp.vz[q] = src.vz[j];
+  for (long long q = 4 * ((long long)blockIdx.x * blockDim.x + threadIdx.x); q < n;
+       q += 4ll * gridDim.x * blockDim.x) {
+    float v[5][4];
+    if (q + 4 <= n) {
+      const uint4 j = *reinterpret_cast<const uint4*>(perm + q);
+      const unsigned from[4] = {j.x, j.y, j.z, j.w};
+#pragma unroll
+      for (int k = 0; k < 4; k++) {
+        v[0][k] = src.ox[from[k]];
+        v[1][k] = src.oy[from[k]];
+        v[2][k] = src.vx[from[k]];
+        v[3][k] = src.vy[from[k]];
+        v[4][k] = src.vz[from[k]];
+      }
+      *reinterpret_cast<float4*>(tmp.ox + q) = make_float4(v[0][0], v[0][1], v[0][2], v[0][3]);
+      *reinterpret_cast<float4*>(tmp.oy + q) = make_float4(v[1][0], v[1][1], v[1][2], v[1][3]);
+      *reinterpret_cast<float4*>(tmp.vx + q) = make_float4(v[2][0], v[2][1], v[2][2], v[2][3]);
+      *reinterpret_cast<float4*>(tmp.vy + q) = make_float4(v[3][0], v[3][1], v[3][2], v[3][3]);
+      *reinterpret_cast<float4*>(tmp.vz + q) = make_float4(v[4][0], v[4][1], v[4][2], v[4][3]);
+    } else {
+      for (long long m = q; m < n; m++) {
+        const unsigned j = perm[m];
+        tmp.ox[m] = src.ox[j];
+        tmp.oy[m] = src.oy[j];
+        tmp.vx[m] = src.vx[j];
+        tmp.vy[m] = src.vy[j];
+        tmp.vz[m] = src.vz[j];
+      }
+    }
   }
 }
 
-__global__ void k_copy_mixed(MixedSoA tmp, MixedSoA dst, const long long* __restrict__ d_n) {
+__global__ void __launch_bounds__(PART_THREADS) k_copy_mixed(MixedSoA tmp, MixedSoA dst, const long long* __restrict__ d_n) {
   const long long n = *d_n;
-  for (long long q = (long long)blockIdx.x * blockDim.x + threadIdx.x; q < n; q += (long long)gridDim.x * blockDim.x) {
-    dst.cell[q] = tmp.cell[q];
-    dst.ox[q] = tmp.ox[q];
-    dst.oy[q] = tmp.oy[q];
-    dst.vx[q] = tmp.vx[q];
-    dst.vy[q] = tmp.vy[q];
-    dst.vz[q] = tmp.vz[q];
+  for (long long q = 4 * ((long long)blockIdx.x * blockDim.x + threadIdx.x); q < n;
+       q += 4ll * gridDim.x * blockDim.x) {
+    if (q + 4 <= n) {
+      const int4 c = *reinterpret_cast<const int4*>(tmp.cell + q);
+      const float4 a = *reinterpret_cast<const float4*>(tmp.ox + q), b = *reinterpret_cast<const float4*>(tmp.oy + q);
+      const float4 u = *reinterpret_cast<const float4*>(tmp.vx + q), v = *reinterpret_cast<const float4*>(tmp.vy + q);
+      const float4 w = *reinterpret_cast<const float4*>(tmp.vz + q);
+      *reinterpret_cast<int4*>(dst.cell + q) = c;
+      *reinterpret_cast<float4*>(dst.ox + q) = a;
+      *reinterpret_cast<float4*>(dst.oy + q) = b;
+      *reinterpret_cast<float4*>(dst.vx + q) = u;
+      *reinterpret_cast<float4*>(dst.vy + q) = v;
+      *reinterpret_cast<float4*>(dst.vz + q) = w;
+    } else {
+      for (long long m = q; m < n; m++) {
+        dst.cell[m] = tmp.cell[m];
+        dst.ox[m] = tmp.ox[m];
+        dst.oy[m] = tmp.oy[m];
+        dst.vx[m] = tmp.vx[m];
+        dst.vy[m] = tmp.vy[m];
+        dst.vz[m] = tmp.vz[m];
+      }
+    }
   }
 }
 
@@ -266,18 +320,21 @@ int launch_sort(cudaStream_t st, const Geom& g, const ParticleRef& p, const long
   const long long E = (long long)RADIX * T;
   const int nscan = (int)((E + SCAN_BLOCK - 1) / SCAN_BLOCK);
   int launches = 0;
-  if (p.mixed) k_sort_keys_mixed<<<grid, PART_THREADS, 0, st>>>(p.m, d_n, sc.keys[0]);
-  else k_sort_keys_fp64<<<grid, PART_THREADS, 0, st>>>(g, p.f, d_n, sc.keys[0]);
-  launches++;
+  if (!p.mixed) {
+    k_sort_keys_fp64<<<grid, PART_THREADS, 0, st>>>(g, p.f, d_n, sc.keys[0]);
+    launches++;
+  }
   const int passes = sort_passes(g.nx * g.ny);
   int cur = 0;
   for (int ps = 0; ps < passes; ps++) {
     const int shift = ps * RADIX_BITS;
-    k_radix_hist<<<T, SORT_T, 0, st>>>(sc.keys[cur], d_n, shift, sc.hist, T);
+    // the mixed form's cells are its keys
+    const unsigned* in = p.mixed && ps == 0 ? reinterpret_cast<const unsigned*>(p.m.cell) : sc.keys[cur];
+    k_radix_hist<<<T, SORT_T, 0, st>>>(in, d_n, shift, sc.hist, T);
     k_scan_local<<<nscan, 1024, 0, st>>>(sc.hist, E, sc.bsum);
     k_scan_top<<<1, 1024, 0, st>>>(sc.bsum, nscan);
     k_scan_add<<<(int)((E + 255) / 256), 256, 0, st>>>(sc.hist, E, sc.bsum);
-    k_radix_scatter<<<T, SORT_T, 0, st>>>(sc.keys[cur], ps ? sc.vals[cur] : nullptr, sc.keys[cur ^ 1],
+    k_radix_scatter<<<T, SORT_T, 0, st>>>(in, ps ? sc.vals[cur] : nullptr, sc.keys[cur ^ 1],
                                           sc.vals[cur ^ 1], d_n, shift, sc.hist, T);
     launches += 5;
     cur ^= 1;
@@ -285,12 +342,13 @@ int launch_sort(cudaStream_t st, const Geom& g, const ParticleRef& p, const long
   if (p.mixed) {
     MixedSoA tmp;
     char* b = static_cast<char*>(sc.tmp);
-    tmp.cell = reinterpret_cast<int*>(b);
-    tmp.ox = reinterpret_cast<float*>(b + 4 * cap);
-    tmp.oy = reinterpret_cast<float*>(b + 8 * cap);
-    tmp.vx = reinterpret_cast<float*>(b + 12 * cap);
-    tmp.vy = reinterpret_cast<float*>(b + 16 * cap);
-    tmp.vz = reinterpret_cast<float*>(b + 20 * cap);
+    const size_t cap4 = 16 * (((size_t)cap + 3) / 4);  // 16-byte aligned arrays; five fit into 24 cap
+    tmp.cell = reinterpret_cast<int*>(sc.keys[cur]);
+    tmp.ox = reinterpret_cast<float*>(b);
+    tmp.oy = reinterpret_cast<float*>(b + cap4);
+    tmp.vx = reinterpret_cast<float*>(b + 2 * cap4);
+    tmp.vy = reinterpret_cast<float*>(b + 3 * cap4);
+    tmp.vz = reinterpret_cast<float*>(b + 4 * cap4);
     k_gather_mixed<<<grid, PART_THREADS, 0, st>>>(p.m, tmp, sc.vals[cur], d_n);
     k_copy_mixed<<<grid, PART_THREADS, 0, st>>>(tmp, p.m, d_n);
   } else {
@@ -310,6 +368,7 @@ int launch_sort(cudaStream_t st, const Geom& g, const ParticleRef& p, const long
 // One buffer: keys x2, vals x2 (4 bytes each per slot), the digit table, the
 // scan totals and the payload copy (payload bytes per slot: 24 for the mixed
 // form's records, 40 for the FP64 form's), each 256-byte aligned.
+
 static size_t al256(size_t b) { return (b + 255) & ~(size_t)255; }
 
 size_t sort_scratch_bytes(long long cap, int payload) {
