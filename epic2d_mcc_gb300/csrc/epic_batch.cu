@@ -571,9 +571,13 @@ __global__ void __launch_bounds__(256) k_batch_spec_residual(BatchSpec b, const 
   spec_residual_chunk(run_lattice(b, e.x), e.y, sm);
 }
 
-__global__ void k_batch_spec_check(BatchSpec b, int nruns, int final_pass) {
-  for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < nruns; r += gridDim.x * blockDim.x)
-    spec_check(run_lattice(b, r), final_pass);
+// A CTA per run (a thread per run, summing its chunks one after the other, took
+// 30 us a stage for 48 runs).
+__global__ void __launch_bounds__(256) k_batch_spec_check(BatchSpec b, int final_pass) {
+  __shared__ int s_e[8];
+  __shared__ unsigned long long s_v[8][2];
+  __shared__ double s_out;
+  spec_check(run_lattice(b, blockIdx.x), final_pass, s_e, s_v, &s_out);
 }
 
 // One of the four products of a refinement stage for every (run, tile) of
@@ -823,12 +827,12 @@ struct epic_batch {
     k_batch_spec_init<<<grid, 256, 0, stream>>>(b, d_node_run, nodes, nruns);
     for (int st = 0; st < BATCH_STAGES; st++) {
       k_batch_spec_residual<<<nchunk, 256, 0, stream>>>(b, chunk_sched);
-      k_batch_spec_check<<<(nruns + 255) / 256, 256, 0, stream>>>(b, nruns, 0);
+      k_batch_spec_check<<<nruns, 256, 0, stream>>>(b, 0);
       for (int prod = 0; prod < 4; prod++)
         for (int w = 0; w < 3; w++) launch_gemms(prod, w);
     }
     k_batch_spec_residual<<<nchunk, 256, 0, stream>>>(b, chunk_sched);
-    k_batch_spec_check<<<(nruns + 255) / 256, 256, 0, stream>>>(b, nruns, 1);
+    k_batch_spec_check<<<nruns, 256, 0, stream>>>(b, 1);
   }
 
   void deposit_all() {
@@ -998,71 +1002,56 @@ epic_status upload_tile_sched(epic_batch* b) {
   return EPIC_OK;
 }
 
-// Times one refinement stage's four products for the runs of each size class
-// with 16-, 32- and 64-wide tiles and keeps the fastest per class (identical
-// results whichever).  Runs before the initial field: it only writes the
-// transform scratch and phi, which every solve starts over.
+// Chooses the product tiles (16, 32 or 64 wide) of each size class by the time
+// of a whole stage's four products over all runs, class after class from 16
+// wide everywhere (identical results whichever).  A class on its own tells
+// less: tiles of one width share a launch, and the launches of different widths
+// follow each other, so a class that would be a tenth faster by itself in wide
+// tiles can cost more than it gains as a launch of its own.  Runs before the
+// initial field: it only writes the transform scratch and phi, which every
+// solve starts over.
 epic_status autotune(epic_batch* b) {
   cudaEvent_t e0, e1;
   cudaEventCreate(&e0);
   cudaEventCreate(&e1);
-  float best[4][3];
-  for (int cls = 0; cls < 4; cls++) best[cls][0] = best[cls][1] = best[cls][2] = 0;
-  const int widths[3] = {16, 32, 64};
-  for (int w = 0; w < 3; w++) {
-    for (int cls = 0; cls < 4; cls++) {
-      bool any = false;
-      for (int r = 0; r < b->nruns; r++) any |= size_class(b->runs[r].R, b->runs[r].C) == cls;
-      if (!any) continue;
-      int saved[4];
-      std::memcpy(saved, b->tiles, sizeof(saved));
-      for (int c = 0; c < 4; c++) b->tiles[c] = 0;  // only this class is scheduled
-      b->tiles[cls] = widths[w];
-      std::vector<int4> by_tile[3];
-      for (int r = 0; r < b->nruns; r++) {
-        const BRun& br = b->runs[r];
-        if (size_class(br.R, br.C) != cls) continue;
-        const int t = b->tiles[cls];
-        for (int tr = 0; tr < (br.R + t - 1) / t; tr++)
-          for (int tc = 0; tc < (br.C + t - 1) / t; tc++) by_tile[w].push_back(make_int4(r, tr, tc, 0));
+  bool any[4] = {};
+  for (int r = 0; r < b->nruns; r++) any[size_class(b->runs[r].R, b->runs[r].C)] = true;
+  epic_status st = EPIC_OK;
+  auto stage_ms = [&](float* ms) -> epic_status {
+    if ((st = upload_tile_sched(b))) return st;
+    auto products = [&] {
+      for (int prod = 0; prod < 4; prod++)
+        for (int w = 0; w < 3; w++) b->launch_gemms(prod, w);
+    };
+    for (int rep = 0; rep < 2; rep++) products();  // warm-up
+    cudaEventRecord(e0, b->stream);
+    for (int rep = 0; rep < 5; rep++) products();
+    cudaEventRecord(e1, b->stream);
+    BCK(cudaEventSynchronize(e1));
+    cudaEventElapsedTime(ms, e0, e1);
+    return EPIC_OK;
+  };
+  for (int cls = 0; cls < 4; cls++)
+    if (any[cls]) b->tiles[cls] = 16;
+  float best = 0;
+  if (!(st = stage_ms(&best))) {
+    for (int cls = 0; cls < 4 && !st; cls++) {
+      if (!any[cls]) continue;
+      int keep = 16;
+      for (int t = 32; t <= 64 && !st; t *= 2) {
+        float ms = 0;
+        b->tiles[cls] = t;
+        if (!(st = stage_ms(&ms)) && ms < best) {
+          best = ms;
+          keep = t;
+        }
       }
-      std::memcpy(b->tiles, saved, sizeof(saved));
-      int4* sc = nullptr;
-      BCK(cudaMallocAsync((void**)&sc, by_tile[w].size() * sizeof(int4), b->stream));
-      BCK(cudaMemcpyAsync(sc, by_tile[w].data(), by_tile[w].size() * sizeof(int4), cudaMemcpyHostToDevice,
-                          b->stream));
-      int4* keep[3] = {b->tile_sched[0], b->tile_sched[1], b->tile_sched[2]};
-      const int nkeep[3] = {b->ntile[0], b->ntile[1], b->ntile[2]};
-      b->tile_sched[0] = b->tile_sched[1] = b->tile_sched[2] = nullptr;
-      b->ntile[0] = b->ntile[1] = b->ntile[2] = 0;
-      b->tile_sched[w] = sc;
-      b->ntile[w] = (int)by_tile[w].size();
-      for (int rep = 0; rep < 2; rep++)
-        for (int prod = 0; prod < 4; prod++) b->launch_gemms(prod, w);  // warm-up
-      cudaEventRecord(e0, b->stream);
-      for (int rep = 0; rep < 5; rep++)
-        for (int prod = 0; prod < 4; prod++) b->launch_gemms(prod, w);
-      cudaEventRecord(e1, b->stream);
-      BCK(cudaEventSynchronize(e1));
-      float ms = 0;
-      cudaEventElapsedTime(&ms, e0, e1);
-      best[cls][w] = ms;
-      cudaFreeAsync(sc, b->stream);
-      for (int k = 0; k < 3; k++) {
-        b->tile_sched[k] = keep[k];
-        b->ntile[k] = nkeep[k];
-      }
+      b->tiles[cls] = keep;
     }
-  }
-  for (int cls = 0; cls < 4; cls++) {
-    if (!(best[cls][0] > 0)) continue;
-    int k = 0;
-    for (int w = 1; w < 3; w++)
-      if (best[cls][w] > 0 && best[cls][w] < best[cls][k]) k = w;
-    b->tiles[cls] = widths[k];
   }
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
+  if (st) return st;
   BCK(cudaGetLastError());
   return upload_tile_sched(b);
 }

@@ -341,10 +341,12 @@ __global__ void __launch_bounds__(PART_THREADS) k_mcc_collide(CrossSections cs, 
   if (threadIdx.x == 0 && s_coll) atomicAdd(&pending[1], s_coll);
 }
 
-// Pass 2 (one block): exclusive scan of the per-tile event counts, 4,096
-// tiles (four per thread) per round.
+// Pass 2 (one block): exclusive scan of the per-tile event counts, 16 tiles a
+// thread and 16,384 a round (a round is one trip to memory and four barriers:
+// 3e5 tiles took 129 us at four a thread).
 __global__ void __launch_bounds__(1024) k_mcc_scan(const long long* __restrict__ d_ne, McEvents ev,
                                                    unsigned long long* pending) {
+  constexpr int SCAN_PER = 16;
   __shared__ unsigned int warp_tot[32];
   __shared__ unsigned int carry;
   const long long ne = *d_ne;
@@ -352,14 +354,22 @@ __global__ void __launch_bounds__(1024) k_mcc_scan(const long long* __restrict__
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   if (threadIdx.x == 0) carry = 0;
   __syncthreads();
-  for (int base = 0; base < tiles; base += 4 * blockDim.x) {
-    const int t0 = base + 4 * threadIdx.x;
-    unsigned int v[4], s = 0;
+  for (int base = 0; base < tiles; base += SCAN_PER * blockDim.x) {
+    const int t0 = base + SCAN_PER * threadIdx.x;
+    unsigned int v[SCAN_PER], s = 0;
+    const bool full = t0 + SCAN_PER <= tiles;
+    if (full) {
 #pragma unroll
-    for (int k = 0; k < 4; k++) {
-      v[k] = t0 + k < tiles ? ev.tile_cnt[t0 + k] : 0u;
-      s += v[k];
+      for (int k = 0; k < SCAN_PER; k += 4) {
+        const uint4 u = *reinterpret_cast<const uint4*>(ev.tile_cnt + t0 + k);
+        v[k] = u.x; v[k + 1] = u.y; v[k + 2] = u.z; v[k + 3] = u.w;
+      }
+    } else {
+#pragma unroll
+      for (int k = 0; k < SCAN_PER; k++) v[k] = t0 + k < tiles ? ev.tile_cnt[t0 + k] : 0u;
     }
+#pragma unroll
+    for (int k = 0; k < SCAN_PER; k++) s += v[k];
     unsigned int x = s;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
@@ -381,9 +391,19 @@ __global__ void __launch_bounds__(1024) k_mcc_scan(const long long* __restrict__
     const unsigned int c0 = carry;
     unsigned int run = c0 + (w ? warp_tot[w - 1] : 0u) + x - s;
 #pragma unroll
-    for (int k = 0; k < 4; k++) {
-      if (t0 + k < tiles) ev.tile_off[t0 + k] = run;
-      run += v[k];
+    for (int k = 0; k < SCAN_PER; k++) {
+      const unsigned int c = v[k];
+      v[k] = run;
+      run += c;
+    }
+    if (full) {
+#pragma unroll
+      for (int k = 0; k < SCAN_PER; k += 4)
+        *reinterpret_cast<uint4*>(ev.tile_off + t0 + k) = make_uint4(v[k], v[k + 1], v[k + 2], v[k + 3]);
+    } else {
+#pragma unroll
+      for (int k = 0; k < SCAN_PER; k++)
+        if (t0 + k < tiles) ev.tile_off[t0 + k] = v[k];
     }
     __syncthreads();  // every thread has read carry and warp_tot
     if (threadIdx.x == blockDim.x - 1) carry = run;

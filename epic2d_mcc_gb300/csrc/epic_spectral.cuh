@@ -15,18 +15,8 @@
 
 namespace epic {
 
-// Exact sum of v[0..n) rounded once (epic_xsum.cuh), by one thread: the
-// batched solve's per-run test.
-__device__ __forceinline__ double spec_exact_sum_serial(const double* v, int n) {
-  int A = 0;
-  for (int b = 0; b < n; b++) A = max(A, xs_exponent(__ldcg(&v[b])));
-  xs_int acc = 0;
-  for (int b = 0; b < n; b++) acc += xs_from_double(__ldcg(&v[b]), A);
-  return xs_to_double(acc, A);
-}
-
-// The same sum by a whole CTA of 256 threads (the same value: exact, then
-// rounded once), in every thread; s_e and s_v: shared scratch of 8 entries.
+// Exact sum of v[0..n) rounded once (epic_xsum.cuh), by a CTA of 256 threads,
+// in every thread; s_e and s_v: shared scratch of 8 entries.
 __device__ __forceinline__ double spec_exact_sum_cta(const double* v, int n, int* s_e, unsigned long long (*s_v)[2],
                                                      double* s_out) {
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
@@ -187,10 +177,13 @@ __device__ __forceinline__ void spec_record(const SpecLattice& L, int done, int 
   }
 }
 
-__device__ __forceinline__ void spec_check(const SpecLattice& L, int final_pass) {
+// By a CTA of 256 threads; s_e, s_v, s_out: as spec_exact_sum_cta.
+__device__ __forceinline__ void spec_check(const SpecLattice& L, int final_pass, int* s_e, unsigned long long (*s_v)[2],
+                                           double* s_out) {
   if (L.state[0]) return;
   const int nchunks = (L.R * L.C + SPEC_CHUNK - 1) / SPEC_CHUNK;
-  const double s = spec_exact_sum_serial(L.partials, nchunks);
+  const double s = spec_exact_sum_cta(L.partials, nchunks, s_e, s_v, s_out);
+  if (threadIdx.x) return;
   double norm, err;
   spec_norm(L, s, norm, err);
   spec_record(L, norm < L.tol, final_pass, err);
