@@ -485,8 +485,6 @@ struct epic_sim {
   double* host_in = nullptr;
   double* host_out = nullptr;
   long long* h_counts = nullptr;  // pinned
-  char* pin = nullptr;            // pinned: the error flags and a call's small results
-  int asks = 0;                   // calls that waited, while there is none
   size_t host_stage_doubles = 0;
   int num_sms;
   int part_grid;
