@@ -1660,6 +1660,7 @@ epic_status epic_batch_get_particles(epic_batch* b, int run, int s, double* out,
       k_batch_to_aos<<<b->grid, PART_THREADS, 0, b->stream>>>(b->runs[run], b->staging, b->arena[s],
                                                                b->poff[(size_t)run * b->nsp + s], cnt);
       BCK(cudaGetLastError());
+      touch_pages(out, (size_t)cnt * 5 * sizeof(double));
       BCK(cudaMemcpyAsync(out, b->staging, (size_t)cnt * 5 * sizeof(double), cudaMemcpyDeviceToHost, b->stream));
     }
     BCK(cudaStreamSynchronize(b->stream));
@@ -1691,6 +1692,7 @@ epic_status epic_batch_get_particles(epic_batch* b, int run, int s, double* out,
   k_batch_gather_run<<<tiles, 256, 0, b->stream>>>(b->runs[run], run, b->d_node_run, b->arena[s], b->d_n[s], d_counts,
                                                    d_out);
   BCK(cudaGetLastError());
+  touch_pages(out, (size_t)total * 5 * sizeof(double));
   if (total) BCK(cudaMemcpyAsync(out, d_out, (size_t)total * 5 * sizeof(double), cudaMemcpyDeviceToHost, b->stream));
   cudaFreeAsync(d_out, b->stream);
   cudaFreeAsync(d_counts, b->stream);
@@ -1703,6 +1705,7 @@ epic_status epic_batch_get_grid(epic_batch* b, int run, int which, double* out) 
   const double* src = which == EPIC_GRID_PHI ? b->phi : which == EPIC_GRID_RHO ? b->rho : nullptr;
   if (!src) return bfail(EPIC_ERR_INVALID, "batches keep phi and rho");
   const BRun& r = b->runs[run];
+  touch_pages(out, (size_t)r.nx * r.ny * sizeof(double));
   BCK(cudaMemcpyAsync(out, src + r.node_off, (size_t)r.nx * r.ny * sizeof(double), cudaMemcpyDeviceToHost,
                       b->stream));
   BCK(cudaStreamSynchronize(b->stream));

@@ -22,6 +22,9 @@
 // the total does not depend on the order the GPU adds them in — used to show
 // that a run's result is bit-identical whether it ran alone or beside others.
 #include <cuda_runtime.h>
+#include <unistd.h>
+
+#include <algorithm>
 
 #include "epic_device.cuh"
 #include "epic_internal.cuh"
@@ -168,6 +171,20 @@ __global__ void k_digest(const void* __restrict__ a, int elem_bytes, const long 
 void launch_digest(cudaStream_t st, const void* a, int elem_bytes, const long long* d_n, long long n,
                    unsigned long long tag, unsigned long long* out, int grid) {
   k_digest<<<grid, PART_THREADS, 0, st>>>(a, elem_bytes, d_n, n, tag, out);
+}
+
+void touch_pages(void* out, size_t bytes) {
+  if (bytes <= 64 * 1024) return;
+  cudaPointerAttributes at;
+  if (cudaPointerGetAttributes(&at, out) != cudaSuccess) {
+    cudaGetLastError();
+    return;
+  }
+  if (at.type != cudaMemoryTypeUnregistered) return;
+  static const long page = std::max(4096l, sysconf(_SC_PAGESIZE));
+  volatile char* const p = static_cast<volatile char*>(out);
+  for (size_t k = 0; k < bytes; k += page) p[k] = p[k];
+  p[bytes - 1] = p[bytes - 1];
 }
 
 }  // namespace epic
