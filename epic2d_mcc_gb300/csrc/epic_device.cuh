@@ -89,39 +89,79 @@ __device__ __forceinline__ bool mcc_candidate(const SelectArgs& s, long long q, 
 // order through an atomic counter, so every tile a block waits on belongs to a
 // block that is already running; each wait is bounded by `limit` polls.
 // status[t] = (state << 62) | value, state 1 = tile aggregate, 2 = inclusive
-// prefix.  Called by one thread; returns the exclusive prefix of `tile`, or
-// ~0 on timeout (FLAG_TIMEOUT set).
+// prefix.  Called by one whole warp; returns the exclusive prefix of `tile` in
+// every lane, or ~0 on timeout (FLAG_TIMEOUT set).
+//
+// A wave of blocks claims its tiles together, so hundreds of tiles may lie
+// between a tile and the last known prefix: the lanes read 32 of them at a
+// time (one after the other each is a trip to L2: the compacting pushes of mixed
+// runs of 64 to 256 cells a side took 48 us on average, 31 so).
 static __device__ unsigned long long tile_lookback(unsigned long long* status, int tile, unsigned long long count,
                                                    int* flags, long long limit) {
-  const unsigned long long MASK = (1ull << 62) - 1;
-  if (tile == 0) {
+  constexpr unsigned long long MASK = (1ull << 62) - 1;
+  const int lane = threadIdx.x & 31;
+  if (lane == 0) {
     __threadfence();
-    atomicExch(&status[0], (2ull << 62) | count);
-    return 0;
+    atomicExch(&status[tile], ((tile == 0 ? 2ull : 1ull) << 62) | count);
   }
-  __threadfence();
-  atomicExch(&status[tile], (1ull << 62) | count);
+  if (tile == 0) return 0;
   unsigned long long prefix = 0;
-  int t = tile - 1;
   long long spins = 0;
-  while (t >= 0) {
-    unsigned long long v = *((volatile unsigned long long*)&status[t]);
-    unsigned long long st = v >> 62;
-    if (st == 0) {
+  for (int t = tile - 1;;) {
+    const int at = t - lane;
+    const unsigned long long v = at >= 0 ? *((volatile unsigned long long*)&status[at]) : 0ull;
+    const unsigned known = __ballot_sync(0xffffffffu, v >> 63);           // an inclusive prefix
+    const unsigned open = __ballot_sync(0xffffffffu, (v >> 62) == 0);     // nothing yet, or before the first tile
+    const int last = known ? __ffs(known) - 1 : 31;
+    if (open & (0xffffffffu >> (31 - last))) {
       if (++spins >= limit) {
-        set_flag(flags, FLAG_TIMEOUT);
+        if (lane == 0) set_flag(flags, FLAG_TIMEOUT);
         return ~0ull;
       }
       __nanosleep(32);
       continue;
     }
-    prefix += v & MASK;
-    if (st == 2) break;
-    t--;
+    // aggregates are at most SCAN_TILE each
+    prefix += __reduce_add_sync(0xffffffffu, lane < last + !known ? (unsigned)v : 0u);
+    if (known) {
+      prefix += __shfl_sync(0xffffffffu, v, last) & MASK;
+      break;
+    }
+    t -= 32;
   }
-  __threadfence();
-  atomicExch(&status[tile], (2ull << 62) | (prefix + count));
+  if (lane == 0) {
+    __threadfence();
+    atomicExch(&status[tile], (2ull << 62) | (prefix + count));
+  }
   return prefix;
+}
+
+// Ranks of a tile's kept particles in row order (row k: the block's threads, in
+// order) by ballots and one barrier; returns their number.  sm: ITEMS x warps
+// entries, free again after the block's next barrier.
+template <int ITEMS>
+static __device__ __forceinline__ int tile_ranks(const int (&keep)[ITEMS], int (&rank)[ITEMS], int* sm) {
+  constexpr int W = PART_THREADS / 32;
+  static_assert(ITEMS * W == 32, "a lane per row and warp");
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  unsigned mask[ITEMS];
+#pragma unroll
+  for (int k = 0; k < ITEMS; k++) {
+    mask[k] = __ballot_sync(0xffffffffu, keep[k]);
+    if (lane == 0) sm[k * W + wid] = __popc(mask[k]);
+  }
+  __syncthreads();
+  const int v = sm[lane];
+  int x = v;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int y = __shfl_up_sync(0xffffffffu, x, o);
+    if (lane >= o) x += y;
+  }
+#pragma unroll
+  for (int k = 0; k < ITEMS; k++)
+    rank[k] = __shfl_sync(0xffffffffu, x - v, k * W + wid) + __popc(mask[k] & ((1u << lane) - 1));
+  return __shfl_sync(0xffffffffu, x, 31);
 }
 
 // Block-wide exclusive scan of one int per thread (PART_THREADS threads).

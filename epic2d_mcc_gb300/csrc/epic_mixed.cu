@@ -405,14 +405,11 @@ __global__ void __launch_bounds__(PART_THREADS) k_push_mixed_compact(Geom g, Mix
       }
     }
     int rank[ITEMS];
-    int tile_total = 0;
-#pragma unroll
-    for (int k = 0; k < ITEMS; k++) {
-      int row_total;
-      rank[k] = tile_total + block_exclusive_scan(keep[k], &row_total, sm);
-      tile_total += row_total;
+    const int tile_total = tile_ranks(keep, rank, sm);
+    if (threadIdx.x < 32) {
+      const unsigned long long before = tile_lookback(status, tile, (unsigned long long)tile_total, flags, spin);
+      if (threadIdx.x == 0) s_prefix = before;
     }
-    if (threadIdx.x == 0) s_prefix = tile_lookback(status, tile, (unsigned long long)tile_total, flags, spin);
     __syncthreads();
     const unsigned long long prefix = s_prefix;
     if (prefix != ~0ull) {
