@@ -126,6 +126,23 @@ struct MixedParticles {
   }
 };
 
+// Whether mcc_collide would surely find "no collision" for these velocities and
+// the first draw u0, in FP32: with the logarithmic table in shared memory, an
+// energy within half an entry of the true one bounds the cross section by the
+// three entries around it, and 1 - exp(-x) <= x.  The margins (1e-4 of x; u0
+// beyond 1e-11, five orders above the rounding of 1 - exp) cover every rounding
+// on the way, so only draws that the exact test rejects too are reported.
+__device__ __forceinline__ bool mcc_surely_none(const CrossSections& cs, const MccParams& m, float vx, float vy, float vz,
+                                                double u0) {
+  if (cs.kind != 1 || !cs.stab || m.null_collision || cs.n < 3 || !(cs.inv_dlog < 1000)) return false;
+  const float v = sqrtf(vx * vx + vy * vy + vz * vz) * (float)m.vn;
+  const float e = fminf(fmaxf((float)(0.5 * ME / EV) * v * v, (float)cs.e_min), (float)cs.e_max);
+  const float u = (logf(e) - (float)cs.log_emin) * (float)cs.inv_dlog;
+  const int i = min(max((int)floorf(u - 0.5f), 0), (int)cs.n - 3);
+  const float tot = __double2float_ru(fmax(fmax(cs.stab[i].x, cs.stab[i + 1].x), cs.stab[i + 2].x));
+  return (float)u0 > 1e-11f && (float)u0 > 1.0001f * (tot * v * (float)m.dt_phys);
+}
+
 // CollisionHandler::handle_collisions for one electron plus collision_electron
 // (src/collision.cpp:60-207), after its first draw u0 passed the early-out
 // below; later draws come from `src` in the reference's order.  Returns 0
@@ -652,6 +669,7 @@ __global__ void __launch_bounds__(PART_THREADS) k_batch_mcc_collide(CrossSection
                                                                     int* flags) {
   extern __shared__ double4 s_tab[];
   __shared__ unsigned long long s_coll;
+  __shared__ unsigned int s_left, s_list[PART_THREADS];
   const unsigned int nc = *ev.cand_count;
   if ((unsigned long long)blockIdx.x * blockDim.x >= nc) return;  // no candidates for this CTA
   if (threadIdx.x == 0) s_coll = 0;
@@ -659,26 +677,45 @@ __global__ void __launch_bounds__(PART_THREADS) k_batch_mcc_collide(CrossSection
   __syncthreads();
   const unsigned long long step = *d_step;
   unsigned int ncoll = 0;
-  for (unsigned int c = blockIdx.x * blockDim.x + threadIdx.x; c < nc; c += gridDim.x * blockDim.x) {
-    const long long q = ev.cand[c];
-    const BRun& r = runs[node_run[e.p.cell[q]]];
-    const MccParams m = batch_mcc_params(r);
-    IonEvent evt;
-    Philox src{(uint32_t)q, (uint32_t)(q >> 32), (uint32_t)step, (uint32_t)r.seed, (uint32_t)(r.seed >> 32), 0,
-               make_uint4(0, 0, 0, 0)};
-    const unsigned long long M = src.next53();
-    const int kind = mcc_collide(cs, m, e, q, src, (double)M * (1.0 / 9007199254740992.0), evt);
-    ncoll += kind != 0;
-    if (kind == 3) {
-      unsigned int slot = atomicAdd(ev.count, 1u);
-      if (slot < ev.cap) {
-        ev.buf[slot] = evt;
-        ev.slot[q] = (int)slot;
-        atomicAdd(&ev.tile_cnt[q / MCC_TILE], 1u);
-      } else {
-        set_flag(flags, FLAG_CAPACITY);
+  for (unsigned int c0 = blockIdx.x * blockDim.x; c0 < nc; c0 += gridDim.x * blockDim.x) {
+    // A candidate's draw is below its run's largest collision probability, and
+    // most are above their own: these go first, the rest share full warps of the
+    // FP64 path.
+    if (threadIdx.x == 0) s_left = 0;
+    __syncthreads();
+    const unsigned int c = c0 + threadIdx.x;
+    if (c < nc) {
+      const long long q = ev.cand[c];
+      const BRun& r = runs[node_run[e.p.cell[q]]];
+      Philox src{(uint32_t)q, (uint32_t)(q >> 32), (uint32_t)step, (uint32_t)r.seed, (uint32_t)(r.seed >> 32), 0,
+                 make_uint4(0, 0, 0, 0)};
+      const double u0 = (double)src.next53() * (1.0 / 9007199254740992.0);
+      if (!mcc_surely_none(cs, batch_mcc_params(r), e.p.vx[q], e.p.vy[q], e.p.vz[q], u0))
+        s_list[atomicAdd(&s_left, 1u)] = (unsigned int)q;
+    }
+    __syncthreads();
+    if (threadIdx.x < s_left) {
+      const long long q = s_list[threadIdx.x];
+      const BRun& r = runs[node_run[e.p.cell[q]]];
+      const MccParams m = batch_mcc_params(r);
+      IonEvent evt;
+      Philox src{(uint32_t)q, (uint32_t)(q >> 32), (uint32_t)step, (uint32_t)r.seed, (uint32_t)(r.seed >> 32), 0,
+                 make_uint4(0, 0, 0, 0)};
+      const unsigned long long M = src.next53();
+      const int kind = mcc_collide(cs, m, e, q, src, (double)M * (1.0 / 9007199254740992.0), evt);
+      ncoll += kind != 0;
+      if (kind == 3) {
+        unsigned int slot = atomicAdd(ev.count, 1u);
+        if (slot < ev.cap) {
+          ev.buf[slot] = evt;
+          ev.slot[q] = (int)slot;
+          atomicAdd(&ev.tile_cnt[q / MCC_TILE], 1u);
+        } else {
+          set_flag(flags, FLAG_CAPACITY);
+        }
       }
     }
+    __syncthreads();  // s_left and s_list are rewritten
   }
   if (ncoll) atomicAdd(&s_coll, (unsigned long long)ncoll);
   __syncthreads();
