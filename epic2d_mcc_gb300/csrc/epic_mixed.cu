@@ -137,8 +137,11 @@ void launch_deposit_mixed_range(cudaStream_t st, const Geom& g, const MixedSoA& 
 // equal addresses queue up as well.  Here a CTA owns a band of rows, holds its
 // node words in shared memory, goes through its slice of all particles, keeps
 // those of its band, and adds the words to the grid once at the end.  Bands
-// are as few as 220 KB a CTA allow: each particle is looked at once per band,
-// and only reading it (12 bytes, from L2 after the first band) is repeated.
+// are as few as 204 KB a CTA allow: each particle is looked at once per band,
+// and only reading it (12 bytes, from L2 after the first band) is repeated;
+// those of the band are queued so that whole warps deposit (without, the
+// atomics of three bands ran a third full: push and deposit of the 256 x 256
+// beam 275 us a step, 260 with).
 //
 // A word is two 32-bit halves, the low one added with the old value returned,
 // which tells the carry: shared memory has no 64-bit add, and its emulation as
@@ -150,7 +153,9 @@ void launch_deposit_mixed_range(cudaStream_t st, const Geom& g, const MixedSoA& 
 constexpr int DT_THREADS = 1024;
 constexpr int DT_PER_THREAD = 8;  // consecutive particles a thread, loaded as vectors
 constexpr int DT_CHUNK = DT_THREADS * DT_PER_THREAD;
-constexpr int DT_MAX_SMEM = 220 * 1024;
+constexpr int DT_QUEUE = 64;  // records a warp
+constexpr int DT_QUEUES = DT_THREADS / 32 * DT_QUEUE * 8;  // 16 KB
+constexpr int DT_MAX_SMEM = 204 * 1024;  // of words
 
 __device__ __forceinline__ void dt_add(unsigned* lo, unsigned* hi, int k, unsigned long long w) {
   const unsigned l = (unsigned)w, old = atomicAdd(lo + k, l);
@@ -158,6 +163,9 @@ __device__ __forceinline__ void dt_add(unsigned* lo, unsigned* hi, int k, unsign
 }
 
 // Band b: cell rows [b rows, (b + 1) rows), node rows one more.
+// QUEUE (several bands): a warp's particles of its band wait in a queue of its
+// own until 32 are there, as one 64-bit record each.
+template <bool QUEUE>
 __global__ void __launch_bounds__(DT_THREADS, 1) k_deposit_mixed_bands(Geom g, MixedSoA p,
                                                                        const long long* __restrict__ d_n,
                                                                        unsigned long long* __restrict__ acc, int bands,
@@ -174,6 +182,17 @@ __global__ void __launch_bounds__(DT_THREADS, 1) k_deposit_mixed_bands(Geom g, M
   unsigned* const lo = dt_words;
   unsigned* const hi = dt_words + words;
   for (int k = threadIdx.x; k < 2 * words; k += DT_THREADS) dt_words[k] = 0;
+  const int lane = threadIdx.x & 31;
+  // past the words of a whole band, 8-byte aligned
+  unsigned long long* const queue =
+      reinterpret_cast<unsigned long long*>(dt_words + 2 * (rows + 1) * g.ny) + (threadIdx.x >> 5) * DT_QUEUE;
+  int waiting = 0;
+  auto deposit = [&](int m, unsigned a, unsigned b) {
+    dt_add(lo, hi, m, (unsigned long long)(S - a) * (S - b));
+    dt_add(lo, hi, m + g.ny, (unsigned long long)a * (S - b));
+    dt_add(lo, hi, m + 1, (unsigned long long)(S - a) * b);
+    dt_add(lo, hi, m + g.ny + 1, (unsigned long long)a * b);
+  };
   __syncthreads();
   for (long long chunk = (long long)slice * DT_CHUNK; chunk < n; chunk += (long long)slices * DT_CHUNK) {
     const long long q0 = chunk + (long long)threadIdx.x * P;
@@ -201,13 +220,31 @@ __global__ void __launch_bounds__(DT_THREADS, 1) k_deposit_mixed_bands(Geom g, M
 #pragma unroll
     for (int k = 0; k < P; k++) {
       const int m = c[k] - c0;
-      if ((unsigned)m < (unsigned)span) {
-        const unsigned a = (unsigned)(int)(ox[k] * fS), b = (unsigned)(int)(oy[k] * fS);
-        dt_add(lo, hi, m, (unsigned long long)(S - a) * (S - b));
-        dt_add(lo, hi, m + g.ny, (unsigned long long)a * (S - b));
-        dt_add(lo, hi, m + 1, (unsigned long long)(S - a) * b);
-        dt_add(lo, hi, m + g.ny + 1, (unsigned long long)a * b);
+      const bool in = (unsigned)m < (unsigned)span;
+      const unsigned a = (unsigned)(int)(ox[k] * fS), b = (unsigned)(int)(oy[k] * fS);
+      if (!QUEUE) {
+        if (in) deposit(m, a, b);
+        continue;
       }
+      const unsigned mask = __ballot_sync(0xffffffffu, in);
+      if (in)
+        queue[waiting + __popc(mask & ((1u << lane) - 1))] =
+            (unsigned long long)m << 40 | (unsigned long long)a << 20 | b;
+      waiting += __popc(mask);
+      if (waiting >= 32) {
+        __syncwarp();
+        waiting -= 32;
+        const unsigned long long v = queue[waiting + lane];
+        __syncwarp();
+        deposit((int)(v >> 40), (unsigned)(v >> 20) & (S - 1), (unsigned)v & (S - 1));
+      }
+    }
+  }
+  if (QUEUE) {
+    __syncwarp();
+    if (lane < waiting) {
+      const unsigned long long v = queue[lane];
+      deposit((int)(v >> 40), (unsigned)(v >> 20) & (S - 1), (unsigned)v & (S - 1));
     }
   }
   __syncthreads();
@@ -217,7 +254,7 @@ __global__ void __launch_bounds__(DT_THREADS, 1) k_deposit_mixed_bands(Geom g, M
   }
 }
 
-// Grids of up to eight bands' words (475 x 475 nodes) whose rows are short
+// Grids of up to eight bands' words (457 x 457 nodes) whose rows are short
 // enough that a band has several.  Measured over whole steps: 400 x 400 cells
 // (six bands) 1.06 to 1.1 times as fast as the fused push and deposit, 256 x
 // 256 1.2, 128 x 128 2; with few particles (4 a cell) level.
@@ -234,9 +271,11 @@ void launch_deposit_mixed_bands(cudaStream_t st, const Geom& g, const MixedSoA& 
   int dev = 0, sms = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  const int smem = (rows + 1) * g.ny * 8;
-  cudaFuncSetAttribute(k_deposit_mixed_bands, cudaFuncAttributeMaxDynamicSharedMemorySize, DT_MAX_SMEM);
-  k_deposit_mixed_bands<<<bands * std::max(1, sms / bands), DT_THREADS, smem, st>>>(g, p, d_n, acc, bands, rows);
+  const int smem = (rows + 1) * g.ny * 8 + (bands > 1 ? DT_QUEUES : 0);
+  const auto kern = bands > 1 ? k_deposit_mixed_bands<true> : k_deposit_mixed_bands<false>;
+  // the same value whatever the grid: other threads may be launching it too
+  cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, DT_MAX_SMEM + DT_QUEUES);
+  kern<<<bands * std::max(1, sms / bands), DT_THREADS, smem, st>>>(g, p, d_n, acc, bands, rows);
 }
 
 // -------------------------------------------------------------- push ---

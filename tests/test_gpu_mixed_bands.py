@@ -22,7 +22,8 @@ def _sim(E, ini, parts, sort_every):
 @pytest.mark.parametrize("nx,ny,n,bc,crowd", [
     (5, 5, 1, "pbc", False), (16, 24, 8191, "reflective", False), (60, 33, 8193, "pbc", False),
     (64, 64, 200001, "pbc", True), (166, 168, 30000, "pbc", False), (168, 166, 30007, "open", False),
-    (250, 301, 300005, "reflective", False), (474, 473, 60001, "pbc", False), (480, 476, 60001, "pbc", False)])
+    (250, 301, 300005, "reflective", False), (456, 455, 60001, "pbc", False), (474, 473, 60001, "pbc", False),
+    (480, 476, 60001, "pbc", False)])
 def test_bands_equal_sorted_deposit(gpu_lib, tmp_path, nx, ny, n, bc, crowd):
     E = gpu_lib
     ini = decks.write(decks.deck(nx=nx, ny=ny, ne=n, ni=n, bc=bc, solver="cg", tol="1e-8", maxit=100000), str(tmp_path))
