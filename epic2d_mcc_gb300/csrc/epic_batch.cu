@@ -187,7 +187,8 @@ struct RunNy {
 };
 
 // T threads per CTA (128 or 256; the autotuner picks the shape), each taking
-// DEP_PER_THREAD consecutive particles per round.
+// DEP_PER_THREAD particles per round in groups of four consecutive ones, as
+// k_push_mixed_dep.
 template <bool SEL, int T>
 __global__ void __launch_bounds__(T, 768 / T) k_batch_push_dep(const BRun* __restrict__ runs,
                                                                     const int* __restrict__ node_run, MixedSoA p,

@@ -152,7 +152,7 @@ __device__ __forceinline__ bool push_mixed_one(const Geom& g, const FieldCell* _
 // ------------------------------------------ deposit of a sorted chunk ---
 // CIC deposit (integer weights, Domain::Scatter, src/domain.cpp:205-228) of a
 // warp's DEP_WARP_CHUNK consecutive particles, sorted by cell (or nearly so,
-// between sorts), DEP_PER_THREAD consecutive particles per lane.
+// between sorts), DEP_PER_THREAD particles per lane, neighbours together.
 //
 // A particle's weights come from its offsets quantised to 2^-20 of a cell,
 // a, b in [0, S), S = 2^20: (S-a)(S-b), a(S-b), (S-a)b, ab on the cell's four
