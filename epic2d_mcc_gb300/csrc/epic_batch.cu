@@ -1250,6 +1250,7 @@ epic_status build(epic_batch* b, const epic_request* reqs, int nruns) {
     const double cell_area = c.dx * c.dy;
     const double L2 = c.L * c.L;
     br.div = cell_area * L2 * c.density;
+    br.rdiv = known_divisor(br.div, br.spwt, b->nsp);
     br.inv_scale = std::ldexp(1.0, -2 * MIXED_OFFSET_BITS);
     br.K = (c.L * c.L) / (c.LDe * c.LDe);
     br.tol = c.tolerance;

@@ -16,7 +16,7 @@ struct BRun {
   double x0, y0, dx, dy;
   float qmK_dt[BATCH_MAX_SPECIES], hqmK_dt[BATCH_MAX_SPECIES], cx, cy;
   double spwt[BATCH_MAX_SPECIES], charge_over_qe[BATCH_MAX_SPECIES];
-  double div, inv_scale, K, tol;
+  double div, rdiv, inv_scale, K, tol;
   // spectral lattice: R x C entries at lat_off of the lattice pools, its
   // transforms at qR_off / qC_off of the transform pool, D at lat_off
   int R, C, flat, gs_norm;

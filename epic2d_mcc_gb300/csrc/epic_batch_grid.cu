@@ -22,7 +22,7 @@ __global__ void k_batch_finalize(BatchGrids b) {
       const unsigned long long* acc = b.acc[s] + r.node_off;
       auto raw = [&](int ii, int jj) {
         const double v = ((double)(long long)acc[ii * ny + jj] * r.inv_scale) * r.spwt[s];
-        return v / r.div;
+        return divide_known(v, r.div, r.rdiv);
       };
       const double v = fold_density(r.bc, nx, ny, raw, i, j);
       const double t = v * r.charge_over_qe[s];

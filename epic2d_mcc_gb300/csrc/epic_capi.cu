@@ -382,6 +382,7 @@ FinalizeArgs finalize_args(epic_sim* s, int stage, int only) {
     a.charge_over_qe[k] = sp.desc.charge * (1 / QE);
     a.active[k] = only < 0 || only == k;
   }
+  a.rdiv = a.fixed ? known_divisor(a.div, a.spwt, a.nsp) : 0;
   a.rho = s->rho;
   return a;
 }

@@ -40,7 +40,7 @@ __device__ __forceinline__ double raw_den(const FinalizeArgs& a, int s, int i, i
   double v;
   if (a.fixed) v = ((double)(long long)a.acc[s][k] * a.inv_scale[s]) * a.spwt[s];
   else v = reinterpret_cast<const double*>(a.acc[s])[k];
-  return v / a.div;
+  return divide_known(v, a.div, a.rdiv);
 }
 
 

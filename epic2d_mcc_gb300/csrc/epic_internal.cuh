@@ -16,6 +16,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <cmath>
 #include <string>
 #include <vector>
 
@@ -363,6 +364,15 @@ void launch_particle_sums(cudaStream_t st, int what, const SoA& p, const long lo
 // FINALIZE_AND_RHO: every species, then rho; RHO_FROM_DEN: rho from the
 // already finalised density grids.
 enum { FINALIZE_ONLY = 0, FINALIZE_AND_RHO = 1, RHO_FROM_DEN = 2 };
+// RN(1/d) for divide_known, or 0 where d or a dividend's scale is so extreme
+// (or not finite) that its product or remainder could leave the normal range.
+inline double known_divisor(double d, const double* scale, int n) {
+  auto plain = [](double x) { return x != 0 && std::fabs(x) > 0x1p-300 && std::fabs(x) < 0x1p300; };
+  for (int k = 0; k < n; k++)
+    if (!plain(scale[k])) return 0;
+  return plain(d) ? 1.0 / d : 0;
+}
+
 struct FinalizeArgs {
   Geom g;
   int nsp;
@@ -370,7 +380,7 @@ struct FinalizeArgs {
   int fixed;
   int stage;
   int active[8];
-  double div;
+  double div, rdiv;  // rdiv: known_divisor
   const unsigned long long* acc[8];
   double* den[8];
   double spwt[8];
