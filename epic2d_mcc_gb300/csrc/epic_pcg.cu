@@ -162,7 +162,9 @@ __device__ __forceinline__ double pmf_double(PmF a, bool neg) {
 // ~1,500 (measured, 16 and 152 CTAs).  Global words are first polled PM_DELAY
 // cycles after the own ones are written: polls in flight while the others'
 // words arrive hold them up (152 CTAs: 3,700 cycles polled at once, 1,500 after
-// 200 to 400).
+// 200 to 400).  Whole iterations, first poll after 250, 400, 475, 550 cycles:
+// 129 x 129 2.01, 1.88, 1.80, 1.84 us; 98 x 145 1.95, 1.86, 1.81, 1.85; 257 x 256
+// 1.82, 1.82, 1.84, 1.88; 1024 x 1024 periodic 2.48, 2.49, 2.51, 2.55.
 //
 // Anchors: against the biased exponent E of the last total, a term with biased
 // exponent e is its significand times 2^(6 + e - E), rounded, so the last total
