@@ -224,7 +224,7 @@ int64_t epic_estimate_bytes(const epic_config* c, const epic_species_desc* sp, i
   const bool mixed = c->precision == EPIC_PRECISION_MIXED;
   int64_t b = N * 8 * (4 + 2 + 8) + N * 16 * nsp;  // phi rho efx efy, ef, 8 solver vectors, den + acc
   if (mixed) {
-    b += N * 8;                                                            // ef32
+    b += N * 8;  // ef32 (4 doubles a node) for ef and one solver vector
     b += 3 * N * 4 + ((int64_t)c->nx * c->nx + (int64_t)c->ny * c->ny) * 4;  // spectral D, scratch, transforms
   }
   int64_t cmax = 0, nmax = 0;
