@@ -29,7 +29,18 @@ namespace epic {
 
 constexpr int SRW_T = 512;                  // threads: the row warps, and all of them for a residual
 constexpr int SRW_ROWS = 256;               // rows: two warps per quarter of the SM
+constexpr int SRW_CHECK = 25;               // residual after sweeps 0, 25, 50, ... (src/field.cpp:118)
 constexpr size_t SRW_SMEM = 200 * 1024;
+
+// Steps between the starts of two sweeps, and of one sweep from its first row's
+// first node to past its last row's last.
+struct SorRowsPeriod {
+  int P, D;
+};
+__host__ __device__ inline SorRowsPeriod sor_rows_period(bool per, int nxi, int nyi) {
+  const int row_warps = (nxi + 31) >> 5, chain = nxi + row_warps;
+  return {per && chain > nyi ? chain : nyi, chain - 1 + nyi - 1};
+}
 
 // PER: columns wrap too (EPIC_POISSON_PERIODIC).  phi: rows of ld >= nyi + 2
 // nodes, ld - 1 odd, so that the lanes' nodes of a step (one row and one column
@@ -43,7 +54,8 @@ __global__ void __launch_bounds__(SRW_T) k_sor_rows(SolverArgs a, int ld) {
   const int i0 = PER ? 0 : 1, nxi = nx - 1 - i0, nyi = ny - 1, ni = nxi * nyi;
   const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int row_warps = (nxi + 31) >> 5;
-  const int P = PER ? max(nxi + row_warps, nyi) : nyi, D = nxi + row_warps - 1 + nyi - 1;
+  const SorRowsPeriod pd = sor_rows_period(PER, nxi, nyi);
+  const int P = pd.P, D = pd.D;
   double* const src = a.work[1];   // rho K, minus its mean when periodic
   double* const snap = a.work[0];  // the checked sweep
   auto node = [&](int q) { return (i0 + q / nyi) * ny + q % nyi; };
@@ -95,7 +107,7 @@ __global__ void __launch_bounds__(SRW_T) k_sor_rows(SolverArgs a, int ld) {
   double edge = 0;                                    // and, in lane 0, its W
   int j = -1 - row - wid;       // node of this step (j < 0: not yet, j >= nyi: between sweeps)
   int left = a.max_iter;        // sweeps to do
-  constexpr int CHECK = 25;     // residual after sweeps 0, 25, 50, ... (src/field.cpp:118)
+  constexpr int CHECK = SRW_CHECK;
   int to_check = real ? 0 : -1; // sweeps to the next checked one
   int iter = 0, converged = 0;
   double L2 = 0;
@@ -171,7 +183,10 @@ __global__ void __launch_bounds__(SRW_T) k_sor_rows(SolverArgs a, int ld) {
 }
 
 // The wrapping lattices that one CTA holds, with unit cells; false otherwise.
-// (The extensions have at least 5 x 5 nodes, epic_create.)
+// (The extensions have at least 5 x 5 nodes, epic_create.)  There is one
+// snapshot: a checked sweep must end, D steps after its start, before the first
+// row is at the next one, CHECK sweeps or CHECK P steps after it.  Lattices with
+// walls and about 25 times as many rows as nodes a row are beyond that.
 bool launch_sor_rows(cudaStream_t st, const SolverArgs& a) {
   if (a.poisson_bc == EPIC_POISSON_DIRICHLET || a.g.dx != 1.0 || a.g.dy != 1.0) return false;
   const bool per = a.poisson_bc == EPIC_POISSON_PERIODIC;
@@ -179,6 +194,8 @@ bool launch_sor_rows(cudaStream_t st, const SolverArgs& a) {
   const int ld = (nyi + 3) & ~1;
   const size_t smem = (size_t)((nxi + 31) / 32 * 32 + 1) * ld * sizeof(double);
   if (nxi < 3 || nyi < 4 || nxi > SRW_ROWS || smem > SRW_SMEM) return false;
+  const SorRowsPeriod pd = sor_rows_period(per, nxi, nyi);
+  if (pd.D - 1 >= SRW_CHECK * pd.P) return false;
   static std::atomic<bool> ready{false};
   if (!ready.load()) {
     cudaFuncSetAttribute(k_sor_rows<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SRW_SMEM);
