@@ -223,7 +223,11 @@ bool launch_sor_rows(cudaStream_t st, const SolverArgs& a) {
 // ring of messages and is three steps old, which hides the way (~300 cycles)
 // behind a step.  A word of a message that has not come yet holds a NaN that no
 // operation gives (SST_NONE), so the readers poll the words that they need, and
-// set them back after the step.  No phi lies in memory at all while the sweeps
+// set them back after the step; the sender may use them again once the reader
+// has counted the step as done (credit, every SST_LOOK steps; released by the
+// reader and acquired by the sender, with fences on shared memory alone: whole
+// ones would wait for the snapshots' stores too and took 4 % of a conductor
+// deck's solve).  No phi lies in memory at all while the sweeps
 // run.  (Splitting rows
 // over the cluster, k_sor_cluster, needs values from both neighbours every step,
 // and spent 2 us on it, most of it in the cluster barrier.)
@@ -268,6 +272,15 @@ __device__ __forceinline__ void sst_put(unsigned addr, int v) {
 __device__ __forceinline__ int sst_get(const int* p) {
   int v;
   asm volatile("ld.volatile.shared::cta.u32 %0, [%1];" : "=r"(v) : "r"(sst_smem(p)) : "memory");
+  return v;
+}
+// Of the word that lets the sweeps write a snapshot that has been read.
+__device__ __forceinline__ void sst_put_release(unsigned addr, int v) {
+  asm volatile("st.release.cluster.shared::cluster.u32 [%0], %1;" ::"r"(addr), "r"(v) : "memory");
+}
+__device__ __forceinline__ int sst_get_acquire(const int* p) {
+  int v;
+  asm volatile("ld.acquire.cluster.shared::cta.u32 %0, [%1];" : "=r"(v) : "r"(sst_smem(p)) : "memory");
   return v;
 }
 __device__ __forceinline__ double sst_ld(unsigned addr) {
@@ -358,7 +371,7 @@ __global__ void __launch_bounds__(SST_T) k_sor_stream(SolverArgs a, SorStream t)
           sst_put(sst_map(&s_out[0], threadIdx.x), 1);
           sst_put(sst_map(&s_cmd, threadIdx.x), 1);
         } else {
-          sst_put(sst_map(&s_checked, threadIdx.x), k + 1);
+          sst_put_release(sst_map(&s_checked, threadIdx.x), k + 1);
         }
       }
       if (threadIdx.x == 0 && conv) {
@@ -485,6 +498,7 @@ __global__ void __launch_bounds__(SST_T) k_sor_stream(SolverArgs a, SorStream t)
         long long tries = 0;
         while (sst_get(&s_credit) < n + SST_LOOK - 1 - t.depth + Pn && sst_get(&s_cmd) == 0)
           if (++tries >= spin) s_cmd = 2;
+        asm volatile("fence.acquire.sync_restrict::shared::cluster.cluster;" ::: "memory");
       }
       if (threadIdx.x == 0) s_stop[look] = sst_get(&s_cmd);
       for (int left = SST_LOOK; left > 0;) {
@@ -501,7 +515,7 @@ __global__ void __launch_bounds__(SST_T) k_sor_stream(SolverArgs a, SorStream t)
               while (sst_get(&s_checked) <= k - SST_SNAPS && sst_get(&s_cmd) == 0)
                 if (++tries >= spin) s_cmd = 2;
               __syncwarp();
-              on_cur = sst_get(&s_checked) > k - SST_SNAPS;
+              on_cur = sst_get_acquire(&s_checked) > k - SST_SNAPS;
             }
             dst_cur = a.work[1 + k % SST_SNAPS];
           } else if (s == a.max_iter - 1) {
@@ -526,7 +540,10 @@ __global__ void __launch_bounds__(SST_T) k_sor_stream(SolverArgs a, SorStream t)
       }
       if (s_stop[look]) break;
       // all but the last step's words are set back, and before a barrier
-      if (threadIdx.x == 0) sst_put(prev_credit, n - 1);
+      if (threadIdx.x == 0) {
+        asm volatile("fence.release.sync_restrict::shared::cta.cluster;" ::: "memory");
+        sst_put(prev_credit, n - 1);
+      }
     }
     if (sst_get(&s_cmd) == 2 && threadIdx.x == 0) atomicOr(a.flags, FLAG_TIMEOUT);
   }
