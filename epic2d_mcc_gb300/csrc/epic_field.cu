@@ -588,17 +588,22 @@ __global__ void __launch_bounds__(SORC_THREADS) k_sor_cluster(SolverArgs a, int 
   cl.sync();  // no CTA leaves while another may still read its band
 }
 
-// Whether the device can co-schedule a cluster of C CTAs of this kernel with
-// this shared memory (asked once per kernel, size and shared memory).
-static bool cluster_fits(const void* kern, int C, int threads, size_t smem) {
+// Sets what a launch of this kernel as one cluster of C CTAs needs; whether the
+// device can co-schedule it with this shared memory.  The attributes belong to
+// the current device's context and are set for every launch (another device, or
+// the same one after a reset, would not have them); the answer does not change,
+// so each device is asked once per kernel, size and shared memory.
+bool cluster_fits(const void* kern, int C, int threads, size_t smem, size_t smem_max) {
   static std::mutex mu;
-  static std::map<std::tuple<const void*, int, size_t>, bool> known;
+  static std::map<std::tuple<int, const void*, int, int, size_t>, bool> known;
+  int dev = 0;
+  cudaGetDevice(&dev);
+  cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_max);
+  cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
   std::lock_guard<std::mutex> lock(mu);
-  const auto key = std::make_tuple(kern, C, smem);
+  const auto key = std::make_tuple(dev, kern, C, threads, smem);
   const auto f = known.find(key);
   if (f != known.end()) return f->second;
-  cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SOR_SMEM_MAX);
-  cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
   cudaLaunchConfig_t cfg = {};
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -658,7 +663,7 @@ static SorCluster sor_cluster_shape(const SolverArgs& a) {
     with_rk = 0;
   }
   const size_t smem = band * (1 + with_rk + k);
-  if (!cluster_fits((const void*)k_sor_cluster<FLUID, UNIT, EXT>, C, SORC_THREADS, smem)) return c;
+  if (!cluster_fits((const void*)k_sor_cluster<FLUID, UNIT, EXT>, C, SORC_THREADS, smem, SOR_SMEM_MAX)) return c;
   c.C = C;
   c.R = R;
   c.with_rk = with_rk;
@@ -684,19 +689,16 @@ static bool launch_sor_cluster(cudaStream_t st, const SolverArgs& a) {
   cfg.stream = st;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, k_sor_cluster<FLUID, UNIT, EXT>, a, c.R, c.with_rk, c.K) == cudaSuccess;
+  return launched(cudaLaunchKernelEx(&cfg, k_sor_cluster<FLUID, UNIT, EXT>, a, c.R, c.with_rk, c.K));
 }
 
 void init_field_kernels() {
-  static bool done = false;
-  if (done) return;
   cudaFuncSetAttribute(k_sor_lex<false, false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SOR_SMEM_MAX);
   cudaFuncSetAttribute(k_sor_lex<false, true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SOR_SMEM_MAX);
   cudaFuncSetAttribute(k_sor_lex<true, false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SOR_SMEM_MAX);
   cudaFuncSetAttribute(k_sor_lex<true, true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SOR_SMEM_MAX);
   cudaFuncSetAttribute(k_sor_lex<false, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SOR_SMEM_MAX);
   cudaFuncSetAttribute(k_sor_lex<false, true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SOR_SMEM_MAX);
-  done = true;
 }
 
 static bool sor_unit(const SolverArgs& a) { return a.g.dx == 1.0 && a.g.dy == 1.0; }
@@ -1019,10 +1021,9 @@ void launch_nrpcg(cudaStream_t st, const SolverArgs& a) {
     cfg.numAttrs = 1;
     SolverArgs an = a;
     an.tol_bits = xs_bits(xs_sqrt_threshold(1e-4));  // the cg's stop test, |r| < 1e-4
-    if (cluster_fits((const void*)k_nrpcg_cluster, C, NRC_THREADS, smem) &&
-        cudaLaunchKernelEx(&cfg, k_nrpcg_cluster, an, per) == cudaSuccess)
+    if (cluster_fits((const void*)k_nrpcg_cluster, C, NRC_THREADS, smem, SOR_SMEM_MAX) &&
+        launched(cudaLaunchKernelEx(&cfg, k_nrpcg_cluster, an, per)))
       return;
-    cudaGetLastError();
   }
   k_nrpcg<<<1, 1024, 0, st>>>(a);
 }

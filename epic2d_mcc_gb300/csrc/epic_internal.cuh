@@ -451,7 +451,14 @@ __host__ __device__ inline int lattice_wrap(int v, int n, int wrap) {
 // (node nx-1 from node 0, node ny-1 from node 0) and the zero x walls of
 // DIRICHLET_X (epic_field.cu).
 void launch_fill_poisson_nodes(cudaStream_t st, const Geom& g, int poisson_bc, double* phi);
-void init_field_kernels();  // one-time kernel attributes (called by epic_create)
+void init_field_kernels();  // kernel attributes on the current device (called by epic_create)
+// A launch's outcome where another kernel takes over from a refused one: its
+// error does not stay behind for the next check to find.
+inline bool launched(cudaError_t e) {
+  if (e != cudaSuccess) cudaGetLastError();
+  return e == cudaSuccess;
+}
+bool cluster_fits(const void* kern, int C, int threads, size_t smem, size_t smem_max);  // epic_field.cu
 void set_last_error(const char* msg);  // the message epic_last_error() returns on this thread
 void launch_sor_lex(cudaStream_t st, const SolverArgs& a);
 bool launch_sor_rows(cudaStream_t st, const SolverArgs& a);  // epic_sor.cu

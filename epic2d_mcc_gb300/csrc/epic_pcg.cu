@@ -25,7 +25,6 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
-#include <atomic>
 #include <cmath>
 
 #include "epic_internal.cuh"
@@ -887,24 +886,20 @@ static bool pm_plan(const Lattice& l, int max_blocks, PcgModes* out) {
   return true;
 }
 
+// (the attribute is set for every launch: cluster_fits)
 template <int NPT>
 static bool pm_launch(cudaStream_t st, const SolverArgs& a, const PcgModes& t) {
   const void* kern = (const void*)k_pcg_modes<NPT, false>;
-  static std::atomic<bool> ready{false};
-  if (!ready.load()) {
-    cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, PM_SMEM_MAX);
-    ready.store(true);
-  }
+  cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, PM_SMEM_MAX);
   SolverArgs args = a;
   PcgModes plan = t;
   void* params[] = {&args, &plan};
-  return cudaLaunchCooperativeKernel(kern, dim3(t.B), dim3(PM_ALL), params, t.smem, st) == cudaSuccess;
+  return launched(cudaLaunchCooperativeKernel(kern, dim3(t.B), dim3(PM_ALL), params, t.smem, st));
 }
 
-// False if the device cannot co-schedule the cluster (asked once per size).
+// False if the device cannot co-schedule the cluster.
 static bool pm_launch_cluster(cudaStream_t st, const SolverArgs& a, const PcgModes& t) {
-  const void* kern = (const void*)k_pcg_modes<1, true>;
-  static std::atomic<int> fits[PM_CLUSTER + 1];  // 1 yes, 2 no
+  if (!cluster_fits((const void*)k_pcg_modes<1, true>, t.B, PM_ALL, PM_SMEM_MAX, PM_SMEM_MAX)) return false;
   cudaLaunchConfig_t cfg = {};
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -913,22 +908,11 @@ static bool pm_launch_cluster(cudaStream_t st, const SolverArgs& a, const PcgMod
   attr[0].val.clusterDim.z = 1;
   cfg.gridDim = dim3(t.B);
   cfg.blockDim = dim3(PM_ALL);
-  cfg.dynamicSmemBytes = PM_SMEM_MAX;
+  cfg.dynamicSmemBytes = t.smem;
   cfg.stream = st;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  int f = fits[t.B].load();
-  if (!f) {
-    int nc = 0;
-    cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, PM_SMEM_MAX);
-    cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-    f = cudaOccupancyMaxActiveClusters(&nc, kern, &cfg) == cudaSuccess && nc >= 1 ? 1 : 2;
-    if (f == 2) cudaGetLastError();
-    fits[t.B].store(f);
-  }
-  if (f == 2) return false;
-  cfg.dynamicSmemBytes = t.smem;
-  return cudaLaunchKernelEx(&cfg, k_pcg_modes<1, true>, a, t) == cudaSuccess;
+  return launched(cudaLaunchKernelEx(&cfg, k_pcg_modes<1, true>, a, t));
 }
 
 // Launches the solve (bar[0..1] zeroed on the stream before it); false where

@@ -20,7 +20,6 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
-#include <atomic>
 
 #include "epic_internal.cuh"
 #include "epic_xsum.cuh"
@@ -196,12 +195,8 @@ bool launch_sor_rows(cudaStream_t st, const SolverArgs& a) {
   if (nxi < 3 || nyi < 4 || nxi > SRW_ROWS || smem > SRW_SMEM) return false;
   const SorRowsPeriod pd = sor_rows_period(per, nxi, nyi);
   if (pd.D - 1 >= SRW_CHECK * pd.P) return false;
-  static std::atomic<bool> ready{false};
-  if (!ready.load()) {
-    cudaFuncSetAttribute(k_sor_rows<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SRW_SMEM);
-    cudaFuncSetAttribute(k_sor_rows<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SRW_SMEM);
-    ready.store(true);
-  }
+  const void* kern = per ? (const void*)k_sor_rows<true> : (const void*)k_sor_rows<false>;
+  cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SRW_SMEM);  // of this device
   if (per) k_sor_rows<true><<<1, SRW_T, smem, st>>>(a, ld);
   else k_sor_rows<false><<<1, SRW_T, smem, st>>>(a, ld);
   return true;
@@ -593,7 +588,7 @@ bool launch_sor_stream(cudaStream_t st, const SolverArgs& a_in, bool fluid) {
   SolverArgs a = a_in;
   a.spin = spin_limit();
   const void* kern = fluid ? (const void*)k_sor_stream<true> : (const void*)k_sor_stream<false>;
-  static std::atomic<int> fits[2][SST_CTAS + 1];  // 1 yes, 2 no
+  if (!cluster_fits(kern, t.C + 1, SST_T, SST_SMEM, SST_SMEM)) return false;
   cudaLaunchConfig_t cfg = {};
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -602,25 +597,12 @@ bool launch_sor_stream(cudaStream_t st, const SolverArgs& a_in, bool fluid) {
   attr[0].val.clusterDim.z = 1;
   cfg.gridDim = dim3(t.C + 1);
   cfg.blockDim = dim3(std::max(SST_CHECK_T, 32 * t.Wr * t.slots));
-  cfg.dynamicSmemBytes = SST_SMEM;
+  cfg.dynamicSmemBytes = t.smem;
   cfg.stream = st;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  int f = fits[fluid][t.C + 1].load();
-  if (!f) {
-    int nc = 0;
-    cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SST_SMEM);
-    cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-    cudaLaunchConfig_t big = cfg;
-    big.blockDim = dim3(SST_T);
-    f = cudaOccupancyMaxActiveClusters(&nc, kern, &big) == cudaSuccess && nc >= 1 ? 1 : 2;
-    if (f == 2) cudaGetLastError();
-    fits[fluid][t.C + 1].store(f);
-  }
-  if (f == 2) return false;
-  cfg.dynamicSmemBytes = t.smem;
-  return (fluid ? cudaLaunchKernelEx(&cfg, k_sor_stream<true>, a, t) : cudaLaunchKernelEx(&cfg, k_sor_stream<false>, a, t)) ==
-         cudaSuccess;
+  return launched(fluid ? cudaLaunchKernelEx(&cfg, k_sor_stream<true>, a, t)
+                        : cudaLaunchKernelEx(&cfg, k_sor_stream<false>, a, t));
 }
 
 }  // namespace epic
