@@ -166,18 +166,38 @@ __device__ __forceinline__ double pmf_double(PmF a, bool neg) {
 // 1.82, 1.82, 1.84, 1.88; 1024 x 1024 periodic 2.48, 2.49, 2.51, 2.55.
 //
 // Anchors: against the biased exponent E of the last total, a term with biased
-// exponent e is its significand times 2^(6 + e - E), rounded, so the last total
-// stands at 2^58 and a term is rounded at 2^-59 of it: for 2^15 terms 2^-53 of
-// the sum, FP64's own rounding.  Each sum has its own anchor.  A sum beyond
-// 2^61 (a total that grew eightfold in one step) or a term beyond 2^61 marks the
-// word; the round is then repeated with anchors PM_WIDEN higher, as is the first
-// one with the anchors it has found.  A sum that stays beyond every anchor is
-// not finite: phi is NaN then, as the reference's would be.
+// exponent e is its significand times 2^(6 + e - E), so the last total stands at
+// 2^58.  Terms are rounded PM_FRAC bits below that unit (622,592 of them: half a
+// unit off) and only the words to the unit itself: at most 160 words, evenly
+// spread, are 2^-56 of the last total off (worst case 2^-52), whatever the number
+// of terms.  (Each term rounded to the unit: 2^-54 with 4,000 terms, 2^-50 with
+// 600,000; alpha of 65,000 terms up to 7e-16 off, 6e-17 so.)  A total below a
+// quarter of its anchor has lost two of those bits, and its round is repeated with
+// the anchors it has found.  Each sum has its own anchor.  A sum beyond 2^61 (a
+// total that grew eightfold in one step) or a term beyond 2^61 marks the word; the
+// round is then repeated with anchors PM_WIDEN higher.  A sum that stays beyond
+// every anchor is not finite: phi is NaN then, as the reference's would be.
 constexpr int PM_TOP = 6;
 constexpr int PM_SCALE = -1075 - PM_TOP;  // a sum V against anchor E is V 2^(E + PM_SCALE)
 constexpr int PM_WIDEN = 24;
+constexpr int PM_NARROW = 52;  // lower, where nothing of a total shows
+constexpr int PM_FRAC = 9;
 constexpr int PM_DELAY = 400;
 constexpr unsigned long long PM_OUT = (1ull << 62) - 1;
+
+// A thread's sum against an anchor.
+struct PmSum {
+  unsigned long long v = 0;  // units
+  unsigned f = 0;            // 2^-PM_FRAC of one
+  bool out = false;          // a term or the sum is out of range
+  // m 2^-n units
+  __device__ __forceinline__ void add(unsigned long long m, int n) {
+    const unsigned long long below = xs_shl(m, (unsigned)(64 - n)) | xs_shr(m, (unsigned)(n - 64));
+    v += xs_shr(m, (unsigned)n);
+    f += ((unsigned)(below >> (63 - PM_FRAC)) + 1) >> 1;
+    out |= (m && n < 3) || (v >> 61) != 0;
+  }
+};
 
 // r^2 and L r^2 of a component, added to the sums.  From the significands: a
 // 64 x 64-bit high product takes ~40 cycles of the integer pipe, an FP64 product
@@ -185,28 +205,40 @@ constexpr unsigned long long PM_OUT = (1ull << 62) - 1;
 // taken apart again (an iteration at 257 x 257: 1.89 us with FP64 products,
 // 1.82 us so; with 16 components a thread, 1024 x 1024: 6.8 against 6.0 us).
 // Cut at 2^-62 of the term, where an FP64 product is rounded at 2^-53.
-__device__ __forceinline__ void pm_terms(unsigned long long& v0, unsigned long long& v1, bool& b0, bool& b1, double r,
-                                         double L, int E0, int E1) {
+__device__ __forceinline__ void pm_terms(PmSum& s0, PmSum& s1, double r, double L, int E0, int E1) {
   const unsigned long long b = xs_bits(r), l = xs_bits(L);  // L >= 0
   const int eb = (int)((b >> 52) & 0x7FF), el = (int)(l >> 52);
   const unsigned long long m = eb ? (b << 11) | (1ull << 63) : 0ull;  // |r| = m 2^(eb - 1086); below the normal range: 0
   const unsigned long long lm = el ? (l << 11) | (1ull << 63) : 0ull;
   const unsigned long long p = __umul64hi(m, m), q = __umul64hi(p, lm);  // r^2 = p 2^(2 eb - 2108), L r^2 = q 2^(2 eb + el - 3130)
-  const int n0 = E0 + 1027 - 2 * eb, n1 = E1 + 2049 - 2 * eb - el;      // shifts to the anchors
-  v0 += (xs_shr(p, (unsigned)(n0 - 1)) + 1) >> 1;
-  v1 += (xs_shr(q, (unsigned)(n1 - 1)) + 1) >> 1;
-  b0 |= eb >= 2047 || (m && n0 < 3) || (v0 >> 61) != 0;
-  b1 |= (m && n1 < 3) || (v1 >> 61) != 0;
+  s0.add(p, E0 + 1027 - 2 * eb);  // shifts to the anchors
+  s1.add(q, E1 + 2049 - 2 * eb - el);
+  s0.out |= eb >= 2047;
 }
 
-// Warp total of v <= 2^61 in every lane, saturated to PM_OUT from 2^61 on.
-__device__ __forceinline__ unsigned long long pm_warp_sum(unsigned long long v) {
-  const unsigned M = (1u << 21) - 1;
-  const unsigned l0 = __reduce_add_sync(0xffffffffu, (unsigned)v & M);
-  const unsigned l1 = __reduce_add_sync(0xffffffffu, (unsigned)(v >> 21) & M);
-  const unsigned l2 = __reduce_add_sync(0xffffffffu, (unsigned)(v >> 42));
-  const unsigned long long t = (unsigned long long)l0 + ((unsigned long long)l1 << 21) + ((unsigned long long)l2 << 42);
-  return l2 >> 18 || t >> 61 ? PM_OUT : t;
+// A warp's total in every lane, as three limbs whose sums over the eight warps of
+// a CTA still fit 32 bits: 14 bits of units with the bits below, 24, and the rest
+// (2^23 and more: out of range).
+constexpr int PM_L1 = 14, PM_L2 = PM_L1 + 24;
+template <int NPT>
+__device__ __forceinline__ uint3 pm_warp_sum(const PmSum& s) {
+  unsigned long long v = s.v;
+  unsigned f = s.f;
+  if (NPT > 1) {
+    v += f >> PM_FRAC;
+    f &= (1u << PM_FRAC) - 1;
+  }
+  uint3 l;
+  l.x = __reduce_add_sync(0xffffffffu, (((unsigned)v & ((1u << PM_L1) - 1)) << PM_FRAC) + f);
+  l.y = __reduce_add_sync(0xffffffffu, (unsigned)(v >> PM_L1) & ((1u << 24) - 1));
+  l.z = __reduce_add_sync(0xffffffffu, s.out ? 1u << (61 - PM_L2) : (unsigned)(v >> PM_L2));
+  return l;
+}
+// Limbs as units, rounded; saturated to PM_OUT from 2^61 on.
+__device__ __forceinline__ unsigned long long pm_units(uint3 l) {
+  const unsigned long long t = ((l.x + (1u << (PM_FRAC - 1))) >> PM_FRAC) + ((unsigned long long)l.y << PM_L1) +
+                               ((unsigned long long)l.z << PM_L2);
+  return l.z >> (61 - PM_L2) || t >> 61 ? PM_OUT : t;
 }
 
 __device__ __forceinline__ void pm_store(ulonglong2* p, int half, unsigned long long w) {
@@ -426,7 +458,7 @@ __device__ __forceinline__ void pm_orbit(const PcgModes& t, int a, int c, const 
 template <int NPT, bool CLUSTER>
 __global__ void __launch_bounds__(PM_ALL) k_pcg_modes(SolverArgs a, PcgModes t) {
   extern __shared__ double sm[];
-  __shared__ unsigned long long s_sum[2][PM_W];  // the warps' (r, r) and (r, L r)
+  __shared__ uint4 s_sum[2][PM_W];  // the warps' (r, r) and (r, L r) as limbs
   // one cluster: the words [parity][(r, r), (r, L r)][CTA][warp]
   __shared__ unsigned long long s_word[CLUSTER ? 2 * 2 * PM_CLUSTER * PM_W : 1];
   __shared__ int s_ok, s_it, s_nan, s_e[PM_W + 1];
@@ -513,7 +545,7 @@ __global__ void __launch_bounds__(PM_ALL) k_pcg_modes(SolverArgs a, PcgModes t) 
   emax = (int)__reduce_max_sync(0xffffffffu, (unsigned)emax);
   if (lane == 0 && emax) atomicMax(a.bar + 1, (unsigned)emax);
   if (!barrier()) return;
-  // anchors of the first round: 2^20 of the largest term (which may be
+  // anchors of the first round: far above the largest term (which may be
   // infinite or NaN)
   const int E0 = min((int)__ldcg(a.bar + 1), 2046) + PM_WIDEN;
 
@@ -542,7 +574,6 @@ __global__ void __launch_bounds__(PM_ALL) k_pcg_modes(SolverArgs a, PcgModes t) 
     // (r, L r), in the same instructions.
     const bool odd = lane & 1;
     PmF rrinv{0, 0}, g{0, 0};  // 1/gamma and eta/gamma^2 of the last iteration
-    bool coarse = true;        // the anchors may be far above the totals
     for (;;) {
       const int par = rd & 1;
       const unsigned tag = ((rd >> 1) + 1) & 3u;
@@ -562,14 +593,15 @@ __global__ void __launch_bounds__(PM_ALL) k_pcg_modes(SolverArgs a, PcgModes t) 
       if (!CLUSTER) {
         // the sum of the warps' values: (r, r) in even lanes, (r, L r) in odd
         pm_bar_sync(1);
-        unsigned long long S = 0, any = 0;
+        uint3 l = make_uint3(0, 0, 0);
 #pragma unroll
         for (int k = 0; k < PM_W; k++) {
-          const unsigned long long v = s_sum[odd][k];
-          S += v;
-          any |= v;
+          const uint4 v = s_sum[odd][k];
+          l.x += v.x;
+          l.y += v.y;
+          l.z += v.z;
         }
-        S = (any | S) >> 61 ? PM_OUT : S;
+        const unsigned long long S = pm_units(l);
         if (lane < 2) pm_store(slot + me, lane, (S << 2) | tag);
         const long long c0 = clock64();
         while (clock64() - c0 < PM_DELAY) {
@@ -615,8 +647,10 @@ __global__ void __launch_bounds__(PM_ALL) k_pcg_modes(SolverArgs a, PcgModes t) 
       out = __any_sync(0xffffffffu, out) || lg[2] >> 17 || ld[2] >> 17;
       const PmF gam = pmf_from(lg[0] + ((unsigned long long)lg[1] << 22) + ((unsigned long long)lg[2] << 44), E[0] + PM_SCALE);
       const PmF del = pmf_from(ld[0] + ((unsigned long long)ld[1] << 22) + ((unsigned long long)ld[2] << 44), E[1] + PM_SCALE);
-      const int eg = gam.e + 63 + 1023, ed = del.e + 63 + 1023;
-      const bool again = !late && (out ? E[0] < 4096 : coarse && gam.m);
+      // their exponents; where nothing of them shows, lower ones to look at
+      const int eg = gam.m ? gam.e + 63 + 1023 : E[0] - PM_NARROW, ed = del.m ? del.e + 63 + 1023 : E[1] - PM_NARROW;
+      const bool faint = (eg < E[0] - 2 && E[0] > 0) || (ed < E[1] - 2 && E[1] > 0);
+      const bool again = !late && (out ? E[0] < 4096 : faint);
       const bool nan = out && !again;
       // beta = gamma/gamma_prev (even lanes), gamma^2 (odd lanes)
       const PmF p1 = pmf_mul(gam, odd ? gam : rrinv);
@@ -631,7 +665,6 @@ __global__ void __launch_bounds__(PM_ALL) k_pcg_modes(SolverArgs a, PcgModes t) 
       __syncwarp();
       pm_bar_arrive(2);
       if (again) {
-        coarse = out;
         E[0] = out ? E[0] + PM_WIDEN : eg;
         E[1] = out ? E[1] + PM_WIDEN : ed;
         rd++;
@@ -672,7 +705,6 @@ __global__ void __launch_bounds__(PM_ALL) k_pcg_modes(SolverArgs a, PcgModes t) 
       g = pmf_mul(eta, i2);
       E[0] = eg;
       E[1] = ed;
-      coarse = false;
       it++;
       rd++;
     }
@@ -686,26 +718,22 @@ __global__ void __launch_bounds__(PM_ALL) k_pcg_modes(SolverArgs a, PcgModes t) 
     bool again = true;
     for (;;) {
       const int par = rd & 1;
-      unsigned long long v0 = 0, v1 = 0;
-      bool b0 = false, b1 = false;
+      PmSum s0, s1;
       const double al = again ? 0.0 : s_alpha[par ^ 1];
 #pragma unroll
       for (int j = 0; j < NPT; j++) {
         if (wid * 32 + PM_T * j < t.per) {
           if (!again) r[j] = fma(-al, q[j], r[j]);
-          pm_terms(v0, v1, b0, b1, r[j], L[j], E[0], E[1]);
+          pm_terms(s0, s1, r[j], L[j], E[0], E[1]);
         }
       }
-      v0 = pm_warp_sum(b0 ? 1ull << 61 : v0);
-      v1 = pm_warp_sum(b1 ? 1ull << 61 : v1);
+      const uint3 l0 = pm_warp_sum<NPT>(s0), l1 = pm_warp_sum<NPT>(s1);
+      const uint3 l = lane & 1 ? l1 : l0;
       if (CLUSTER) {
         if (wid < nw && lane < 2 * nb)
-          pm_store_cluster(remote + par * 2 * PM_CLUSTER * PM_W * 8, ((lane & 1 ? v1 : v0) << 2) | (((rd >> 1) + 1) & 3u));
+          pm_store_cluster(remote + par * 2 * PM_CLUSTER * PM_W * 8, (pm_units(l) << 2) | (((rd >> 1) + 1) & 3u));
       } else {
-        if (lane == 0) {
-          s_sum[0][wid] = v0;
-          s_sum[1][wid] = v1;
-        }
+        if (lane < 2) s_sum[lane][wid] = make_uint4(l.x, l.y, l.z, 0);
         __syncwarp();
         pm_bar_arrive(1);
       }
