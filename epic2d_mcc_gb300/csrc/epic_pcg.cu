@@ -801,8 +801,9 @@ __global__ void __launch_bounds__(PM_ALL) k_pcg_modes(SolverArgs a, PcgModes t) 
   if (!barrier()) return;
 
   // domain.error = |A x - b| / n (src/field.cpp:258-259), n = nx ny: each
-  // thread's sum in FP64, the threads' sums added exactly
-  double e2 = 0;
+  // thread's sum in FP64 with what its additions round off beside it, the
+  // threads' sums added exactly
+  double e2 = 0, rest = 0;
   for (int m = me * PM_ALL + threadIdx.x; m < n; m += nb * PM_ALL) {
     const int row = m / C, col = m - row * C;
     const int up = lattice_wrap(row - 1, R, lat.wrap_r), dn = lattice_wrap(row + 1, R, lat.wrap_r);
@@ -814,14 +815,18 @@ __global__ void __launch_bounds__(PM_ALL) k_pcg_modes(SolverArgs a, PcgModes t) 
     if (rt >= 0) sum += __ldcg(&a.phi[lattice_node(lat, row, rt)]);
     if (dn >= 0) sum += __ldcg(&a.phi[lattice_node(lat, dn, col)]);
     const double e = sum - (rhs(row, col) - bmean);
-    e2 = fma(e, e, e2);
+    const double sq = e * e, t = e2 + sq, z = t - e2;
+    rest += (e2 - (t - z)) + (sq - z);
+    e2 = t;
   }
-  emax = (int)__reduce_max_sync(0xffffffffu, (unsigned)xs_exponent(e2));
+  emax = xs_exponent(e2);
+  if (emax == 2047) rest = 0;  // infinite or NaN already
+  emax = (int)__reduce_max_sync(0xffffffffu, (unsigned)emax);
   if (lane == 0) s_e[wid] = emax;
   __syncthreads();
   emax = 0;
   for (int k = 0; k <= PM_W; k++) emax = max(emax, s_e[k]);
-  const xs_int ev = xs_warp_sum(xs_from_double(e2, emax));
+  const xs_int ev = xs_warp_sum(xs_from_double(e2, emax) + xs_from_double(rest, emax));
   if (lane == 0) {
     s_v[wid][0] = (unsigned long long)(xs_uint)ev;
     s_v[wid][1] = (unsigned long long)((xs_uint)ev >> 64);

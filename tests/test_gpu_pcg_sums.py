@@ -1,11 +1,14 @@
-"""The PCG solve's dot products against exact ones.
+"""The PCG solve's sums against exact ones.
 
 Stopped after one iteration from a zero start, phi is -alpha b with alpha = (b, b)/(b, L b), so its projection on b gives
 alpha to below the last bit.  The bound: alpha is rounded once (2^-53).  Each of the two sums crosses the blocks in at most
 160 words rounded to a unit of 2^-58 of the total, evenly spread: sqrt(2 160/12) 2^-58 = 1.8e-17.  What a component of phi
 carries beside it is r's rounding over alpha L, 4/L 2^-53/sqrt(12) of it, which leaves at most 2.2e-17 of the projection on
 these lattices (summed over their eigenvalues).  With 5 sigma of both: 2.6e-16, whatever the number of components.  Sides
-n with n + 1 = 2^odd (walls) and n = 4^k (periodic), where the transforms' scales are exact."""
+n with n + 1 = 2^odd (walls) and n = 4^k (periodic), where the transforms' scales are exact.
+
+Stopped before the first iteration, phi is 0 and the reported error the root of the sum of b^2: large terms first and
+then many that an FP64 sum beside them would lose."""
 import math
 from fractions import Fraction
 
@@ -60,3 +63,19 @@ def test_first_step_length(gpu_lib, tmp_path, nx, ny, wrap):
     sim.close()
     print("first step, %d x %d: off by %s" % (nx, ny, " ".join("%.2e" % o for o in off)))
     assert max(off) <= 2.6e-16
+
+
+@pytest.mark.parametrize("nx,ny", [(60, 61), (1025, 1025)])
+def test_reported_error_is_the_exact_sum(gpu_lib, tmp_path, nx, ny):
+    sim, K = _sim(gpu_lib, tmp_path, nx, ny, 0)
+    rho = np.full((ny, nx), 2.0 ** -27)
+    rho.ravel()[: min(46000, nx * ny // 2)] = 1.0  # beyond every thread's first term
+    rho = rho.ravel()
+    edge = np.zeros((nx, ny), dtype=bool)
+    edge[0] = edge[-1] = edge[:, 0] = edge[:, -1] = True
+    sim.set_grid("rho", rho)
+    it, err, conv = sim.potential_solver()
+    assert it == 0 and not conv and not sim.grid("phi").any()
+    b = np.where(edge.ravel(), 0.0, rho * K)
+    assert err == math.sqrt(math.fsum(b * b)) / (nx * ny)
+    sim.close()
