@@ -70,10 +70,12 @@ long long nnodes(const epic_sim* s) { return (long long)s->cfg.nx * s->cfg.ny; }
 // memory waits for itself, so a value and the flags took three round trips (a
 // step and its diagnostics on 17 x 17 nodes, 16 calls: 0.61 ms, 0.45 so).
 // Page-locking the buffer takes 130 us where a call saves 8, so a state gets it
-// once it has been asked PIN_AFTER times; larger results are copied straight to
-// the caller.
+// once 16 calls have gone without: one that stops right after has lost what it
+// would have saved by then.  Larger results are copied straight to the caller.
+// Locking and giving back may wait for every stream of the device, so a state of
+// the server, beside others in flight, does without (never_pin).
 constexpr size_t PIN_BYTES = 64 * 1024, PIN_HEAD = 64;  // data after the flags
-constexpr int PIN_AFTER = 6;
+constexpr int PIN_AFTER = 16;
 
 void pin_when_asked(epic_sim* s) {
   if (s->pin || s->asks > PIN_AFTER || ++s->asks <= PIN_AFTER) return;
@@ -728,6 +730,7 @@ epic_status do_step(epic_sim* s, int with_collisions, int sort = -1) {
 
 namespace epic {
 void set_last_error(const char* msg) { g_err = msg; }
+void never_pin(epic_sim* s) { s->asks = PIN_AFTER + 1; }
 
 static std::atomic<long long> g_spin_limit{SPIN_LIMIT};
 long long spin_limit() { return g_spin_limit.load(std::memory_order_relaxed); }

@@ -49,5 +49,7 @@ void reference_tables(const epic_config& c, std::vector<double>& tot, std::vecto
 double cs_elastic(double energy, int on);
 double cs_excitation(double energy, int on);
 double cs_ionization(double energy, int on);
+// The state keeps no page-locked buffer for its results (epic_capi.cu).
+void never_pin(epic_sim* s);
 
 }  // namespace epic

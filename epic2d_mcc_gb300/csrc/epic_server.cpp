@@ -16,6 +16,7 @@
 
 #include "../../include/epic2d.h"
 #include "../../include/epic2d_serve.h"
+#include "epic_host.h"
 
 namespace {
 
@@ -99,6 +100,7 @@ struct epic_server {
     const epic_request& q = r->req;
     int st = epic_create(&q.cfg, &r->sim);
     if (st) return st;
+    epic::never_pin(r->sim);
     for (int k = 0; k < q.num_species && !st; k++) st = epic_add_species(r->sim, &q.species[k], nullptr);
     for (int k = 0; k < q.num_conductors && !st; k++) st = epic_add_conductor(r->sim, &q.conductors[k]);
     for (int k = 0; k < q.num_emitters && !st; k++) st = epic_add_emitter(r->sim, &q.emitters[k]);
