@@ -254,28 +254,34 @@ __global__ void __launch_bounds__(DT_THREADS, 1) k_deposit_mixed_bands(Geom g, M
   }
 }
 
-// Grids of up to eight bands' words (457 x 457 nodes) whose rows are short
-// enough that a band has several.  Measured over whole steps: 400 x 400 cells
-// (six bands) 1.06 to 1.1 times as fast as the fused push and deposit, 256 x
-// 256 1.2, 128 x 128 2; with few particles (4 a cell) level.
-bool deposit_bands_fit(const Geom& g) {
-  constexpr int per = DT_MAX_SMEM / 8;
-  return g.ny <= per / 8 && (long long)g.nx * g.ny <= 8ll * per;
+// Bands of so many cell rows each that their words, with one row of nodes more,
+// fit a CTA; none is empty.
+struct DepositBands {
+  int rows, bands;
+};
+static DepositBands deposit_bands(const Geom& g) {
+  const int most = DT_MAX_SMEM / 8 / g.ny - 1;  // cell rows that fit
+  const int want = (g.nx - 1 + most - 1) / most, rows = (g.nx - 1 + want - 1) / want;
+  return {rows, (g.nx - 1 + rows - 1) / rows};
 }
+
+// Grids of up to eight bands (450 x 450 nodes) whose rows are short enough that a
+// band has several.  Measured over whole steps: 400 x 400 cells (seven bands) 1.06
+// to 1.1 times as fast as the fused push and deposit, 256 x 256 1.2, 128 x 128 2;
+// with few particles (4 a cell) level.
+bool deposit_bands_fit(const Geom& g) { return g.ny <= DT_MAX_SMEM / 8 / 8 && deposit_bands(g).bands <= 8; }
 
 void launch_deposit_mixed_bands(cudaStream_t st, const Geom& g, const MixedSoA& p, const long long* d_n,
                                 unsigned long long* acc) {
-  const int most = DT_MAX_SMEM / 8 / g.ny - 1;  // cell rows that fit
-  const int want = (g.nx - 1 + most - 1) / most, rows = (g.nx - 1 + want - 1) / want;
-  const int bands = (g.nx - 1 + rows - 1) / rows;  // none is empty
+  const DepositBands b = deposit_bands(g);
   int dev = 0, sms = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  const int smem = (rows + 1) * g.ny * 8 + (bands > 1 ? DT_QUEUES : 0);
-  const auto kern = bands > 1 ? k_deposit_mixed_bands<true> : k_deposit_mixed_bands<false>;
+  const int smem = (b.rows + 1) * g.ny * 8 + (b.bands > 1 ? DT_QUEUES : 0);
+  const auto kern = b.bands > 1 ? k_deposit_mixed_bands<true> : k_deposit_mixed_bands<false>;
   // the same value whatever the grid: other threads may be launching it too
   cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, DT_MAX_SMEM + DT_QUEUES);
-  kern<<<bands * std::max(1, sms / bands), DT_THREADS, smem, st>>>(g, p, d_n, acc, bands, rows);
+  kern<<<b.bands * std::max(1, sms / b.bands), DT_THREADS, smem, st>>>(g, p, d_n, acc, b.bands, b.rows);
 }
 
 // -------------------------------------------------------------- push ---
