@@ -161,9 +161,9 @@ __device__ __forceinline__ double pmf_double(PmF a, bool neg) {
 // ~1,500 (measured, 16 and 152 CTAs).  Global words are first polled PM_DELAY
 // cycles after the own ones are written: polls in flight while the others'
 // words arrive hold them up (152 CTAs: 3,700 cycles polled at once, 1,500 after
-// 200 to 400).  Whole iterations, first poll after 250, 400, 475, 550 cycles:
-// 129 x 129 2.01, 1.88, 1.80, 1.84 us; 98 x 145 1.95, 1.86, 1.81, 1.85; 257 x 256
-// 1.82, 1.82, 1.84, 1.88; 1024 x 1024 periodic 2.48, 2.49, 2.51, 2.55.
+// 200 to 400).  Whole iterations, first poll after 350, 400, 475, 525 cycles:
+// 129 x 129 2.07, 1.93, 1.87, 1.86 us; 98 x 145 2.04, 1.88, 1.86, 1.87; 257 x 256
+// 1.81, 1.85, 1.87, 1.90; 1024 x 1024 periodic 2.52, 2.55, 2.56, 2.60.
 //
 // Anchors: against the biased exponent E of the last total, a term with biased
 // exponent e is its significand times 2^(6 + e - E), so the last total stands at
@@ -203,7 +203,8 @@ struct PmSum {
 // 64 x 64-bit high product takes ~40 cycles of the integer pipe, an FP64 product
 // holds the warp's quarter of the SM for 64 and its result would have to be
 // taken apart again (an iteration at 257 x 257: 1.89 us with FP64 products,
-// 1.82 us so; with 16 components a thread, 1024 x 1024: 6.8 against 6.0 us).
+// 1.82 us with these, before the sums kept the bits below the unit, 1.85 now;
+// with 16 components a thread, 1024 x 1024: 6.8 against 6.0 us).
 // Cut at 2^-62 of the term, where an FP64 product is rounded at 2^-53.
 __device__ __forceinline__ void pm_terms(PmSum& s0, PmSum& s1, double r, double L, int E0, int E1) {
   const unsigned long long b = xs_bits(r), l = xs_bits(L);  // L >= 0

@@ -35,7 +35,8 @@ struct Run {
 
 // Runs admitted alone: those whose FP64 solve is a cooperative launch with one
 // CTA per SM (the PCG, red-black SOR), which would wait for the whole GPU
-// beside other runs.  The mixed form's spectral solve is a cooperative launch
+// beside other runs.  A PCG of up to 4,096 components is one cluster of at most
+// 16 CTAs and would not; it is admitted alone all the same.  The mixed form's spectral solve is a cooperative launch
 // too, sized to its lattice's tiles (at most two CTAs per SM); served runs
 // share the GPU with it.  Every grid-wide wait is bounded (a run whose wait
 // gives up fails with EPIC_ERR_TIMEOUT instead of hanging).
