@@ -162,8 +162,8 @@ __device__ __forceinline__ double pmf_double(PmF a, bool neg) {
 // cycles after the own ones are written: polls in flight while the others'
 // words arrive hold them up (152 CTAs: 3,700 cycles polled at once, 1,500 after
 // 200 to 400).  Whole iterations, first poll after 350, 400, 475, 525 cycles:
-// 129 x 129 2.07, 1.93, 1.87, 1.86 us; 98 x 145 2.04, 1.88, 1.86, 1.87; 257 x 256
-// 1.81, 1.85, 1.87, 1.90; 1024 x 1024 periodic 2.52, 2.55, 2.56, 2.60.
+// 129 x 129 2.08, 1.87, 1.82, 1.85 us; 98 x 145 1.98, 1.86, 1.83, 1.85; 257 x 256
+// 1.80, 1.83, 1.85, 1.88; 1024 x 1024 periodic 2.50, 2.53, 2.55, 2.59.
 //
 // Anchors: against the biased exponent E of the last total, a term with biased
 // exponent e is its significand times 2^(6 + e - E), so the last total stands at
@@ -203,8 +203,7 @@ struct PmSum {
 // 64 x 64-bit high product takes ~40 cycles of the integer pipe, an FP64 product
 // holds the warp's quarter of the SM for 64 and its result would have to be
 // taken apart again (an iteration at 257 x 257: 1.89 us with FP64 products,
-// 1.82 us with these, before the sums kept the bits below the unit, 1.85 now;
-// with 16 components a thread, 1024 x 1024: 6.8 against 6.0 us).
+// 1.82 us so; with 16 components a thread, 1024 x 1024: 6.8 against 6.0 us).
 // Cut at 2^-62 of the term, where an FP64 product is rounded at 2^-53.
 __device__ __forceinline__ void pm_terms(PmSum& s0, PmSum& s1, double r, double L, int E0, int E1) {
   const unsigned long long b = xs_bits(r), l = xs_bits(L);  // L >= 0
@@ -650,7 +649,8 @@ __global__ void __launch_bounds__(PM_ALL) k_pcg_modes(SolverArgs a, PcgModes t) 
       const PmF del = pmf_from(ld[0] + ((unsigned long long)ld[1] << 22) + ((unsigned long long)ld[2] << 44), E[1] + PM_SCALE);
       // their exponents; where nothing of them shows, lower ones to look at
       const int eg = gam.m ? gam.e + 63 + 1023 : E[0] - PM_NARROW, ed = del.m ? del.e + 63 + 1023 : E[1] - PM_NARROW;
-      const bool faint = (eg < E[0] - 2 && E[0] > 0) || (ed < E[1] - 2 && E[1] > 0);
+      // below 2^56 units, a quarter of the anchor (from the limb, beside the chain to beta)
+      const bool faint = (lg[2] < 1u << 12 && E[0] > 0) || (ld[2] < 1u << 12 && E[1] > 0);
       const bool again = !late && (out ? E[0] < 4096 : faint);
       const bool nan = out && !again;
       // beta = gamma/gamma_prev (even lanes), gamma^2 (odd lanes)
